@@ -127,6 +127,10 @@ int mpsxx_context_set_sigma_operator_format(mpsxx_context* ctx, int fp32_operato
  * default (24; 256, for padded sizes shared by at least 6 blocks); 0 switches a route
  * off. */
 int mpsxx_context_set_svd_routes(mpsxx_context* ctx, int jacobi_max_cols, int gram_max_dim);
+/* FP64 H_eff*psi and renormalisations of at least min_flops floating-point operations run
+ * on the tensor cores (error-free slicing, FP64 accuracy), smaller ones on the FP64 pipe;
+ * negative: the default; 0: all on the tensor cores; infinity: none. */
+int mpsxx_context_set_fp64_route(mpsxx_context* ctx, double min_flops);
 /* Plans (H_eff*psi, diagonal, merged-operator, renormalisation) kept per kind before
  * the context empties a cache (default 512).  Plans are keyed by structural layouts,
  * so a converged sweep reuses the previous sweep's plans when they are still cached;

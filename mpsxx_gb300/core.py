@@ -66,6 +66,11 @@ class Context:
         """Wait limit of the tensor-core kernels in ns (<= 0: the default 20 s)."""
         check(lib().mpsxx_context_set_device_timeout(self.h, int(timeout_ns)))
 
+    def set_fp64_route(self, min_flops: float = -1.0):
+        """FP64 products of at least ``min_flops`` run on the tensor cores (error-free
+        slicing), smaller ones on the FP64 pipe; negative: the default, inf: none."""
+        check(lib().mpsxx_context_set_fp64_route(self.h, float(min_flops)))
+
     def set_plan_cache(self, max_plans: int = 512):
         """Plans kept per kind before a cache is emptied."""
         check(lib().mpsxx_context_set_plan_cache(self.h, int(max_plans)))

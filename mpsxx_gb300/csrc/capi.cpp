@@ -1,4 +1,5 @@
 // extern "C" boundary of libmpsxx_gb300 (declared in include/mpsxx_gb300.h).
+#include <cmath>
 #include <cstring>
 #include <exception>
 #include <memory>
@@ -182,6 +183,14 @@ int mpsxx_context_set_device_timeout(mpsxx_context* ctx, int64_t timeout_ns) {
   });
 }
 
+int mpsxx_context_set_fp64_route(mpsxx_context* ctx, double min_flops) {
+  return guard([&] {
+    need(ctx && ctx->ctx, "null context");
+    need(!std::isnan(min_flops), "FP64 route limit is not a number");
+    ctx->ctx->oz_min_flops = min_flops;
+  });
+}
+
 int mpsxx_context_set_plan_cache(mpsxx_context* ctx, int64_t max_plans) {
   return guard([&] {
     need(ctx && ctx->ctx, "null context");
@@ -342,6 +351,7 @@ int mpsxx_tensor_device_ptr(const mpsxx_tensor* t, double** out) {
   return guard([&] {
     need(out != nullptr, "null output");
     *out = ten(t).d;
+    ten(t).exposed = true;
   });
 }
 
@@ -387,7 +397,7 @@ int mpsxx_compute_sigma_vector(mpsxx_context* ctx, const mpsxx_tensor* lopr, con
     need_device(S);
     compute_sigma_vector(c, L, R, P, S);
     c.sync();
-    if (c.precision != kFP64) check_device_error(c);
+    check_device_error(c);
   });
 }
 
@@ -416,7 +426,7 @@ int mpsxx_compute_sigma_vector_onesite(mpsxx_context* ctx, const mpsxx_tensor* m
     need_device(ten(ropr));
     need_device(ten(wfn));
     deliver(ctx, sigma_onesite(c, ten(mpo), ten(lopr), ten(ropr), ten(wfn)), sgv);
-    if (c.precision != kFP64) check_device_error(c);
+    check_device_error(c);
   });
 }
 
@@ -430,7 +440,7 @@ int mpsxx_compute_sigma_vector_twosite(mpsxx_context* ctx, const mpsxx_tensor* l
     need_device(ten(ropr));
     need_device(ten(wfn));
     deliver(ctx, sigma_twosite(c, ten(lmpo), ten(rmpo), ten(lopr), ten(ropr), ten(wfn)), sgv);
-    if (c.precision != kFP64) check_device_error(c);
+    check_device_error(c);
   });
 }
 
@@ -455,6 +465,7 @@ int mpsxx_renormalize_mpo(mpsxx_context* ctx, int forward, const mpsxx_tensor* m
     need_device(ten(bra));
     need_device(ten(ket));
     deliver(ctx, renormalize_mpo(c, forward != 0, ten(mpo), ten(opr0), ten(bra), ten(ket)), opr1);
+    check_device_error(c);
   });
 }
 
@@ -544,6 +555,7 @@ int mpsxx_renormalize(mpsxx_context* ctx, int forward, const mpsxx_tensor* opr0,
     Context& c = ctx_of(ctx);
     auto r = renormalize(c, forward != 0, ten(opr0), ten(bra), ten(ket));
     c.sync();
+    check_device_error(c);
     *opr1 = wrap(std::move(r), ctx);
   });
 }
@@ -636,6 +648,7 @@ int mpsxx_tensor_accumulate(mpsxx_context* ctx, double alpha, const mpsxx_tensor
     DevArray<DCopy> dc;
     dc.upload(cp, c.stream);
     launch_copy(dc.get(), static_cast<int>(cp.size()), X.d, Y.d, 1, c.stream);
+    Y.data_version = next_data_version();  // packed copies of the old data are stale
     c.kernel_launches += 1;
     c.sync();
   });
@@ -684,6 +697,7 @@ int mpsxx_optimize_twosite_merged(mpsxx_context* ctx, int forward, const mpsxx_t
     BondOut b = optimize_twosite_merged(c, forward != 0, ten(lmpo), ten(rmpo), ten(lopr), ten(ropr), ten(lwfn),
                                         ten(rwfn), tole, M, noise);
     c.sync();
+    check_device_error(c);
     if (energy) *energy = b.stats.energy;
     if (stats) {
       stats[0] = b.stats.dav.n_sigma;
@@ -730,6 +744,7 @@ int mpsxx_optimize_twosite_merged_batch(mpsxx_context* ctx, int n, const int* fo
       args[i].noise = noise ? noise[i] : 0.0;
     }
     std::vector<BondOut> out = optimize_twosite_merged_batch(c, args, tole);
+    check_device_error(c);
     for (int i = 0; i < n; ++i) {
       energy[i] = out[i].stats.energy;
       env[i] = wrap(std::move(out[i].env), ctx);
@@ -757,6 +772,7 @@ int mpsxx_mpo_gradient(mpsxx_context* ctx, const mpsxx_tensor* lmpo, const mpsxx
     Context& c = ctx_of(ctx);
     std::vector<double> gl, gr;
     bond_mpo_gradient(c, ten(lmpo), ten(rmpo), ten(lopr), ten(ropr), ten(psi), gl, gr);
+    check_device_error(c);
     std::memcpy(grad_l, gl.data(), gl.size() * sizeof(double));
     std::memcpy(grad_r, gr.data(), gr.size() * sizeof(double));
   });

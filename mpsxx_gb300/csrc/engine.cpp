@@ -281,6 +281,10 @@ template struct DevArray<DCopy>;
 template struct DevArray<DScatterDst>;
 template struct DevArray<DScatterSrc>;
 template struct DevArray<DNoise>;
+template struct DevArray<DOzPack>;
+template struct DevArray<DOzSeg>;
+template struct DevArray<DOzPair>;
+template struct DevArray<DOzTiled>;
 template struct DevArray<double>;
 template struct DevArray<int64_t>;
 template struct DevArray<int>;
@@ -312,8 +316,8 @@ Context::~Context() {
   diag_plans.clear();
   merge_plans.clear();
   renorm_plans.clear();
-  for (DevBuf* b : {&scr1, &scr2, &work, &partial, &scalars, &svd_work, &svd_mats, &gemm_part, &err_flag,
-                    &svd_gram, &svd_gram_work, &svd_ptrs})
+  release_err_flag(*this);
+  for (DevBuf* b : {&scr1, &scr2, &work, &partial, &scalars, &svd_work, &svd_mats, &gemm_part, &svd_gram, &svd_gram_work, &svd_ptrs})
     b->release();
   forget_stream_uploads(stream);
   for (auto& l : svd_lanes) {
@@ -378,8 +382,8 @@ struct CMap {
 
 // Output tiles of every task; the pair list of long tasks is split (split-K) so
 // that a launch fills the GPU: the work of a tile ~ the sum of its pairs' k.
-static void make_tiles(const GemmPlan& plan, int tile_m, int tile_n, std::vector<DTile>& tiles,
-                       std::vector<DReduce>& reduce, int& nslots, int target_ctas = kTargetCtas) {
+void make_tiles(const GemmPlan& plan, int tile_m, int tile_n, std::vector<DTile>& tiles, std::vector<DReduce>& reduce,
+                int& nslots, int target_ctas) {
   tiles.clear();
   reduce.clear();
   nslots = 0;
@@ -445,6 +449,7 @@ static void build_plan_impl(GemmPlan& plan, Trans ta, Trans tb, const Tensor& a,
   plan.h_reduce.clear();
   plan.flops = 0.0;
   plan.c_elems = 0;
+  plan.full = true;
   const int L = a.sh.rank, M = b.sh.rank;
   for (const auto& t : plan.tasks) {
     const CMap c = cmap(t.c_tag);
@@ -494,12 +499,15 @@ static void build_plan_impl(GemmPlan& plan, Trans ta, Trans tb, const Tensor& a,
       plan.flops += 2.0 * double(ma) * double(nb) * double(ka);
     }
     dt.p1 = static_cast<int>(plan.h_pairs.size());
-    if (dt.p1 == dt.p0) continue;
+    if (dt.p1 == dt.p0) {
+      if (c.m > 0 && c.n > 0) plan.full = false;
+      continue;
+    }
     plan.h_tasks.push_back(dt);
     plan.task_ctag.push_back(t.c_tag);
     plan.c_elems += int64_t(c.m) * c.n;
   }
-  make_tiles(plan, kGemmTile, kGemmTile, plan.h_tiles, plan.h_reduce, plan.nslots);
+  make_tiles(plan, kGemmTile, kGemmTile, plan.h_tiles, plan.h_reduce, plan.nslots, kTargetCtas);
   tile_tc(plan, kTargetCtas);
 }
 
@@ -1341,10 +1349,43 @@ static void sigma_run_pk_whole(Context& ctx, SigmaPlan& p, double* sigma) {
   ctx.kernel_launches += 3 + (p.s2.nslots_tc > 0);
 }
 
+// FP64 H_eff * psi on the tensor cores: L psi into the FP64 intermediate (every block has
+// one pair: stacked panels), the intermediate packed, then the sum over w and B'.  The
+// operators' digits are kept while their data stays.  False: no memory for it.
+static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTensor& R, const double* psi,
+                         double* sigma) {
+  {
+    PhaseTimer tm(ctx, kPhSigmaPlan);
+    if (!p.o1.built) build_oz_gemm(ctx, p.o1, p.s1, L, p.psi_layout, true);
+    if (!p.o2.built) build_oz_gemm(ctx, p.o2, p.s2, p.scr1, R, false, &p.o1, &p.s1);
+    if (!oz_reserve(ctx, {&p.o1, &p.o2})) return false;
+    for (auto& x : {std::make_pair(&p.o1.a, &L), std::make_pair(&p.o2.b, &R)}) {
+      OzOperand& o = *x.first;
+      if (o.src_layout == x.second->layout_id && o.src_version == x.second->data_version &&
+          (!x.second->exposed || o.src_call == ctx.call))
+        continue;
+      oz_pack(ctx, o, x.second->d);
+      o.src_layout = x.second->layout_id;
+      o.src_version = x.second->data_version;
+      o.src_call = ctx.call;
+    }
+    tm.stop();
+    ctx.timers[kPhSigma] -= tm.dt;  // counted as planning, not as H_eff * psi
+  }
+  ctx.scr1.ensure(std::max<int64_t>(p.o1.tiled_elems, 1) * sizeof(double), ctx.stream);
+  double* scr = ctx.scr1.as<double>();
+  oz_pack(ctx, p.o1.b, psi);
+  run_oz_gemm(ctx, p.o1, p.s1, 1.0, L.d, psi, scr, true);
+  oz_pack(ctx, p.o2.a, scr);
+  run_oz_gemm(ctx, p.o2, p.s2, 1.0, scr, R.d, sigma, false);
+  return true;
+}
+
 static void sigma_run(Context& ctx, SigmaPlan& p, const DTensor& L, const DTensor& R, const double* psi,
                       double* sigma, int precision) {
   if (precision != kFP64) {
     sigma_run_pk(ctx, p, L, R, psi, sigma);
+  } else if (oz_wanted(ctx, p.flops) && sigma_run_oz(ctx, p, L, R, psi, sigma)) {
   } else {
     ctx.scr1.ensure(std::max<int64_t>(p.scr1.nnz, 1) * sizeof(double), ctx.stream);
     double* scr = ctx.scr1.as<double>();
@@ -1444,23 +1485,62 @@ void apply_sigma(Context& ctx, SigmaPlan& p, const DTensor& L, const DTensor& R,
   sigma_run(ctx, p, L, R, psi, sigma, precision);
 }
 
-// Device error flag of the tensor-core kernels (zeroed on first use).
-int* device_err_flag(Context& ctx) {
-  if (!ctx.err_flag.p) {
-    ctx.err_flag.ensure(sizeof(int), ctx.stream);
-    cuda_check(cudaMemsetAsync(ctx.err_flag.p, 0, sizeof(int), ctx.stream), "err flag zero");
+// Error flags of the tensor-core kernels: one int per context in mapped host memory, which a
+// kernel writes only when it gives up, so that the host reads it without a copy.  The page
+// is never freed; slots are handed out again.
+namespace {
+class ErrSlots {
+ public:
+  int* get() {
+    std::lock_guard<std::mutex> lk(mu_);
+    if (free_.empty()) {
+      int* page = nullptr;
+      cuda_check(cudaHostAlloc(reinterpret_cast<void**>(&page), kSlots * sizeof(int),
+                               cudaHostAllocPortable | cudaHostAllocMapped),
+                 "error flag page");
+      for (int i = 0; i < kSlots; ++i) free_.push_back(page + i);
+    }
+    int* s = free_.back();
+    free_.pop_back();
+    *s = 0;
+    return s;
   }
-  return ctx.err_flag.as<int>();
+  void put(int* s) {
+    std::lock_guard<std::mutex> lk(mu_);
+    free_.push_back(s);
+  }
+
+ private:
+  static constexpr int kSlots = 1024;
+  std::mutex mu_;
+  std::vector<int*> free_;
+};
+ErrSlots& err_slots() {
+  static ErrSlots* e = new ErrSlots;
+  return *e;
+}
+}  // namespace
+
+int* device_err_flag(Context& ctx) {
+  if (!ctx.err_host) {
+    ctx.err_host = err_slots().get();
+    cuda_check(cudaHostGetDevicePointer(reinterpret_cast<void**>(&ctx.err_dev), ctx.err_host, 0), "error flag pointer");
+  }
+  return ctx.err_dev;
+}
+
+void release_err_flag(Context& ctx) {
+  if (ctx.err_host) err_slots().put(ctx.err_host);
+  ctx.err_host = nullptr;
 }
 
 // Throws DEVICE_TIMEOUT when a tensor-core kernel gave up waiting for its MMAs.
 void check_device_error(Context& ctx) {
-  if (!ctx.err_flag.p) return;
-  int h = 0;
-  cuda_check(cudaMemcpyAsync(&h, ctx.err_flag.p, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream), "err d2h");
+  if (!ctx.err_host) return;
   ctx.sync();
-  if (h) {
-    cuda_check(cudaMemsetAsync(ctx.err_flag.p, 0, sizeof(int), ctx.stream), "err flag reset");
+  volatile int* e = ctx.err_host;
+  if (*e) {
+    *e = 0;
     throw Error(kDeviceTimeout, "tensor-core kernel: MMA completion wait timed out");
   }
 }
@@ -1469,12 +1549,14 @@ void compute_sigma_vector(Context& ctx, const DTensor& L, const DTensor& R, cons
   if (sigma.nnz != psi.nnz || sigma.tags != psi.tags)
     throw Error(kInvalidArgument, "compute_sigma_vector: sigma must have the wavefunction's block layout");
   SigmaPlan& p = sigma_plan(ctx, L, R, psi);
+  ++ctx.call;
   sigma_run(ctx, p, L, R, psi.d, sigma.d, ctx.precision);
 }
 
 double sigma_device_time(Context& ctx, const DTensor& L, const DTensor& R, const DTensor& psi, DTensor& sigma,
                          int reps) {
   SigmaPlan& p = sigma_plan(ctx, L, R, psi);
+  ++ctx.call;
   cudaEvent_t e0, e1;
   cuda_check(cudaEventCreate(&e0), "event create");
   cuda_check(cudaEventCreate(&e1), "event create");
@@ -1593,6 +1675,25 @@ RenormPlan& renorm_plan(Context& ctx, bool forward, const Tensor& opr0, const Te
   return insert_plan(ctx, ctx.renorm_plans, key, build_renorm_plan(ctx, forward, opr0, bra, ket));
 }
 
+// Both FP64 contractions on the tensor cores; every operand is new with each call, its
+// digits go back to the block cache afterwards.  False: no memory for it.
+static bool renorm_run_oz(Context& ctx, RenormPlan& rp, const DTensor& bra, const DTensor& opr0, const DTensor& ket,
+                          double* scr, double* out) {
+  if (!rp.o1.built) build_oz_gemm(ctx, rp.o1, rp.p1, conj_view(bra), opr0);
+  if (!rp.o2.built) build_oz_gemm(ctx, rp.o2, rp.p2, rp.scr, ket);
+  if (!oz_reserve(ctx, {&rp.o1, &rp.o2})) return false;
+  oz_pack(ctx, rp.o1.swap ? rp.o1.b : rp.o1.a, bra.d);
+  oz_pack(ctx, rp.o1.swap ? rp.o1.a : rp.o1.b, opr0.d);
+  if (!rp.p1.full) cuda_check(cudaMemsetAsync(scr, 0, rp.scr.nnz * sizeof(double), ctx.stream), "renorm scr zero");
+  run_oz_gemm(ctx, rp.o1, rp.p1, 1.0, bra.d, opr0.d, scr, true);
+  oz_pack(ctx, rp.o2.swap ? rp.o2.b : rp.o2.a, scr);
+  oz_pack(ctx, rp.o2.swap ? rp.o2.a : rp.o2.b, ket.d);
+  run_oz_gemm(ctx, rp.o2, rp.p2, 1.0, scr, ket.d, out, false);
+  rp.o1.release();
+  rp.o2.release();
+  return true;
+}
+
 std::unique_ptr<DTensor> renormalize(Context& ctx, bool forward, const DTensor& opr0, const DTensor& bra,
                                      const DTensor& ket) {
   PhaseTimer tplan(ctx, kPhRenormPlan);
@@ -1612,13 +1713,18 @@ std::unique_ptr<DTensor> renormalize(Context& ctx, bool forward, const DTensor& 
   const int64_t scr_nnz = rp.scr.nnz;
   ctx.scr2.ensure(std::max<int64_t>(scr_nnz, 1) * sizeof(double), ctx.stream);
   double* sp = ctx.scr2.as<double>();
-  if (scr_nnz) cuda_check(cudaMemsetAsync(sp, 0, scr_nnz * sizeof(double), ctx.stream), "renorm scr zero");
+  auto zero_scr = [&] {
+    if (scr_nnz) cuda_check(cudaMemsetAsync(sp, 0, scr_nnz * sizeof(double), ctx.stream), "renorm scr zero");
+  };
   if (split) {
+    zero_scr();
     run_split_gemm(ctx, rp.g1, rp.p1, 1.0, bra.d, opr0.d, sp);
     run_split_gemm(ctx, rp.g2, rp.p2, 1.0, sp, ket.d, out->d);
     for (Packed* P : {&rp.g1.pa, &rp.g1.pb, &rp.g2.pa, &rp.g2.pb}) P->buf.release();
     check_device_error(ctx);
+  } else if (oz_wanted(ctx, rp.p1.flops + rp.p2.flops) && renorm_run_oz(ctx, rp, bra, opr0, ket, sp, out->d)) {
   } else {
+    zero_scr();
     ctx.gemm_part.ensure(std::max(rp.p1.partial_bytes(), rp.p2.partial_bytes()), ctx.stream);
     rp.p1.run(1.0, bra.d, opr0.d, sp, ctx.gemm_part.as<double>(), ctx.stream);
     rp.p2.run(1.0, sp, ket.d, out->d, ctx.gemm_part.as<double>(), ctx.stream);
@@ -2210,6 +2316,7 @@ double normalize_tensor(Context& ctx, DTensor& x) {
   double* sc = ctx.scalars.as<double>();
   launch_multidot(x.d, 1, x.d, 1, n, n, sc + 100, ctx.partial.as<double>(), nblk, ctx.stream);
   launch_scal_dev(x.d, n, sc + 100, 1, ctx.stream);
+  x.data_version = next_data_version();
   ctx.kernel_launches += 3;
   double nrm2 = 0.0;
   cuda_check(cudaMemcpyAsync(&nrm2, sc + 100, sizeof(double), cudaMemcpyDeviceToHost, ctx.stream), "norm d2h");
@@ -2367,7 +2474,12 @@ double diagonalize(Context& ctx, const DTensor& L, const DTensor& R, const DTens
   DavidsonStats local;
   DavidsonStats& S = stats ? *stats : local;
   S = DavidsonStats{};
-  if (ctx.precision == kFP64) return davidson_run(ctx, L, R, diag, wfnc, tol, 0.0, 4, S);
+  ++ctx.call;
+  if (ctx.precision == kFP64) {
+    const double e = davidson_run(ctx, L, R, diag, wfnc, tol, 0.0, 4, S);
+    check_device_error(ctx);
+    return e;
+  }
   // Split precision.  (1) The Davidson iterations with the tensor-core operator, to
   // its resolution.  (2) Refinement: one FP64 H_eff * psi of that vector anchors a
   // continuation of the Davidson run in which only the new correction vectors are
@@ -2411,6 +2523,8 @@ void release_bond_buffers(Context& ctx) {
       P->src_layout = 0;
       P->src_version = ~0ull;
     }
+    kv.second->o1.release();
+    kv.second->o2.release();
     kv.second->group_scr.release();
     kv.second->staged.release();
     kv.second->drop_graph();

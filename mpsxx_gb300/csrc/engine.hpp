@@ -22,6 +22,7 @@ void solver_check(cusolverStatus_t s, const char* what);
 // the block cache serves a new stream (its blocks then wait on events when taken by
 // another stream)
 void register_cache_stream(cudaStream_t st);
+size_t block_cache_bytes();  // held by the block cache for reuse
 
 // Grow-only device buffer.  Storage comes from the process-wide block cache:
 // released blocks are kept for reuse instead of being returned with cudaFree, which
@@ -70,6 +71,9 @@ struct DTensor : Tensor {
   Context* ctx = nullptr;
   DevBuf store;
   std::vector<double> host;  // host copy for MPO coefficients (optional)
+  // the caller holds the device pointer and may write through it unseen: packed copies of
+  // the data last one call
+  mutable bool exposed = false;
   void alloc_device(cudaStream_t st, bool zero = true);
 };
 
@@ -98,6 +102,7 @@ struct GemmPlan {
   int nslots_tc = 0;
   double flops = 0.0;
   int64_t c_elems = 0;  // elements of C touched (for traffic accounting)
+  bool full = true;     // every enumerated task has work (no empty contraction)
   void upload(cudaStream_t st);
   // partial: nslots * 64 * 64 doubles of scratch (may be null when nslots == 0)
   void run(double alpha, const double* A, const double* B, double* C, double* partial, cudaStream_t st) const;
@@ -113,6 +118,17 @@ enum Precision : int { kFP64 = 0, kSplitTF32 = 1, kSplitTF32All = 2 };
 constexpr int kTargetCtas = 152 * 8;
 // packed L*psi intermediates above this size make the tuner try w-blocked schedules
 constexpr int64_t kGroupIntermediateBytes = int64_t(8) << 30;
+
+// sliced FP64 GEMM: output tiles that a plan with long pair lists is split into
+constexpr int kOzTargetTiles = 152 * 8;
+// fewest FLOPs of an FP64 plan that runs sliced on the tensor cores.  One call, FP64 pipe
+// against tensor cores: H_eff*psi 67 : 73 us at 0.18 MFLOP (Hubbard M=32), 96 : 79 at 1.5
+// (M=64), 232 : 87 at 24, 1236 : 158 at 780 (M=512); renormalisation 98 : 94 at 0.24, 123 :
+// 98 at 0.9, 635 : 375 at 4 (QC n=14 M=40); below a megaflop the two more launches of the
+// packing decide.
+constexpr double kOzMinFlops = 1.0e6;
+// packed bytes of a plan that need no look at the free memory (the query is a driver call)
+constexpr int64_t kOzSmallBytes = int64_t(256) << 20;
 
 // plans kept per kind in a context before the cache is emptied
 constexpr size_t kMaxCachedPlans = 512;  // default of Context::max_plans
@@ -148,11 +164,82 @@ struct SplitGemm {
   DevArray<DPkPair> pk;
 };
 
+// One operand of a sliced FP64 GEMM: its digit tiles, row exponents and what they hold.
+struct OzOperand {
+  DevBuf buf, exps;  // exps: one exponent per packed row, then the flag
+  std::vector<int64_t> base;  // per block slot: byte offset of its tile grid (-1: not packed)
+  std::vector<int> exp0, nks;  // per block slot: first exponent, K slices
+  std::vector<DOzPack> h_packs;
+  std::vector<DOzSeg> h_segs;
+  DevArray<DOzPack> packs;
+  DevArray<DOzSeg> segs;
+  int64_t bytes = 0;
+  int rows = 0;
+  int seq = 0;  // packings so far
+  uint64_t src_layout = 0, src_version = ~0ull, src_call = 0;  // what the digits are of
+  void release() {
+    buf.release();
+    exps.release();
+    src_layout = 0;
+    src_version = ~0ull;
+  }
+};
+
+// FP64 execution of one GemmPlan on the tensor cores (kernels_oz.cu).  Tasks of one pair
+// each (a product with a shared small operand: L psi, renormalisations) are run as stacked
+// panels, the rows of all blocks that meet the same block of the shared operand under one
+// another; `swap` makes the plan's B the row operand where A is the shared one.  Longer
+// pair lists run block by block, split along K.
+struct OzGemm {
+  bool built = false, swap = false, stacked = false;
+  OzOperand a, b;  // row operand (128-row tiles) and column operand (32-row tiles)
+  std::vector<DTile> h_tiles;  // by CTA
+  std::vector<int> h_cta_ptr;
+  DevArray<DTile> tiles;
+  DevArray<int> cta_ptr;
+  DevArray<DOzPair> pairs;
+  DevArray<int64_t> row_map;
+  std::vector<DReduce> h_reduce;
+  DevArray<DReduce> reduce;
+  int nslots = 0;
+  // tiled intermediate between two plans: where the first one's tasks go, the size, and
+  // the per-pair places (of the panels, or of the second one's row operand blocks)
+  bool tiled_out = false, tiled_in = false;
+  std::vector<DOzTiled> task_place;
+  int64_t tiled_elems = 0;
+  DevArray<DOzTiled> pairs_tiled;
+  size_t partial_bytes() const { return size_t(nslots) * kOzTileM * kOzTileN * sizeof(double); }
+  int64_t device_bytes() const { return a.bytes + b.bytes + 4 * (int64_t(a.rows) + b.rows); }
+  bool held() const { return a.buf.p && b.buf.p; }
+  void release() {
+    a.release();
+    b.release();
+  }
+};
+// tiled_out: the result goes to a tiled intermediate (stacked, unswapped plans); from: the
+// plan whose tiled result is this one's A (blocks of `a` matched by from's task result tags).
+void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a, const Tensor& b, bool tiled_out = false,
+                   const OzGemm* from = nullptr, const GemmPlan* from_plan = nullptr);
+// Packs an operand of a built plan from FP64 data.
+void oz_pack(Context& ctx, OzOperand& o, const double* src);
+// C = (assign) or += alpha op(A) op(B) from the packed operands.
+void run_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, double alpha, const double* A, const double* B, double* C,
+                 bool assign);
+// Device memory for the plans' packed operands: false (nothing held) when it would take
+// more than half of what is free.
+bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs);
+// whether a plan of that many FLOPs runs on the tensor cores
+bool oz_wanted(const Context& ctx, double flops);
+// Output tiles of every task with long pair lists split along K (engine.cpp)
+void make_tiles(const GemmPlan& plan, int tile_m, int tile_n, std::vector<DTile>& tiles, std::vector<DReduce>& reduce,
+                int& nslots, int target_ctas);
+
 struct SigmaPlan {
   std::mutex pk_mu;  // guards the packed-operand plan (built once, possibly by a planning thread)
   uint64_t l_id = 0, r_id = 0, psi_id = 0;
   Tensor scr1;  // layout of L*psi
   GemmPlan s1, s2;
+  OzGemm o1, o2;  // both stages' FP64 execution on the tensor cores
   double flops = 0.0;
   int64_t bytes_min = 0;  // 8*(nnz L + nnz R + 2 nnz psi)
   // split-TF32 path over packed operands
@@ -237,6 +324,7 @@ struct MergePlan {
 struct RenormPlan {
   Tensor scr, out;
   GemmPlan p1, p2;
+  OzGemm o1, o2;
   bool split_built = false;
   SplitGemm g1, g2;
 };
@@ -307,7 +395,9 @@ struct Context {
   DevBuf svd_work;   // solver workspace
   DevBuf svd_mats;   // per-block SVD matrices
   DevBuf gemm_part;  // split-K partial tiles
-  DevBuf err_flag;   // device error flag of the tensor-core kernels
+  // error flag of the tensor-core kernels (mapped host memory) as the host and the device see it
+  int* err_host = nullptr;
+  int* err_dev = nullptr;
   // canonicalize: independent per-block SVDs run on these lanes concurrently, each
   // driven by its own host thread (the solver's launches are host-bound)
   struct SvdLane {
@@ -336,6 +426,11 @@ struct Context {
   // applies to plans made afterwards
   bool sigma_fp32_operators = false;
   uint64_t device_timeout_ns = kPkTimeoutNs;  // wait limit of the tensor-core kernels
+  // fewest FLOPs of an FP64 plan that runs on the tensor cores (< 0: the default)
+  double oz_min_flops = -1.0;
+  // number of the current product or eigenproblem (a caller's own writes through an exposed
+  // pointer fall between them)
+  uint64_t call = 0;
   // canonicalize routing: blocks with min(m, n) <= svd_jacobi_cols go to the batched
   // Jacobi kernel, the rest with a Gram dimension <= svd_gram_max to the batched
   // eigensolver; < 0 selects the defaults
@@ -414,6 +509,7 @@ SigmaPlan& sigma_plan(Context& ctx, const Tensor& L, const Tensor& R, const Tens
 void compute_sigma_vector(Context& ctx, const DTensor& L, const DTensor& R, const DTensor& psi, DTensor& sigma);
 
 int* device_err_flag(Context& ctx);
+void release_err_flag(Context& ctx);
 void check_device_error(Context& ctx);
 
 // average device seconds of `reps` sigma applications (CUDA events on ctx.stream)

@@ -23,7 +23,8 @@ struct DGemmPair {
 // reduction adds into C (split-K for tasks with long pair lists).
 struct DTile {
   int task, tm, tn, p0, p1, slot;
-  int h64;  // tensor-core tiles: the A rows are a block's 64-row tail tile (see tail64)
+  int h64;  // tensor-core tiles: the A rows are a block's 64-row tail tile (see tail64);
+            // sliced FP64 tiles: the rows of the packed A tile (see oz_tile_rows)
   int nt;   // tensor-core tiles: B rows (output columns) of the tile, 128 or a block's
             // compact tail (see tail_cols)
 };
@@ -165,6 +166,80 @@ void launch_gemm_pk_reduce(const DReduce* red, int nred, const DGemmTask* tasks,
                            double* C, cudaStream_t st);
 void launch_pack(const DPack* packs, int npacks, const double* src, uint8_t* dst, cudaStream_t st);
 int pk_smem_bytes();
+
+// ---- FP64 GEMM on the tensor cores (kernels_oz.cu) ------------------------------
+// Packed digit tiles: A operands in 128-row tiles (a last tile of its rows rounded up to 8:
+// the MMA reads past them into whatever follows, which only reaches rows that nobody reads),
+// B operands (output columns) in 32-row tiles (a last one of at most 16 rows compact); per K
+// slice of 16 the seven digits' rows x 16 bf16.  Padding rows are not written.
+constexpr int kOzTileM = 128, kOzTileN = 32, kOzTileK = 16, kOzDigits = 7;
+constexpr int kOzGroupSteps = 10;     // K slices summed in one FP32 accumulation (exact up to 160)
+constexpr int kOzMaxExponent = 480;   // rows of larger magnitude flag their operand
+constexpr uint32_t kOzTileABytes = kOzDigits * kOzTileM * kOzTileK * 2;
+constexpr uint32_t kOzTileBBytes = kOzDigits * kOzTileN * kOzTileK * 2;
+__host__ __device__ constexpr int oz_tile_rows(int rows, int tm) {
+  return rows - tm * 128 >= 128 ? 128 : (rows - tm * 128 + 7) / 8 * 8;
+}
+__host__ __device__ constexpr int oz_tail_cols(int rows, int tn) {
+  return (tn == rows / 32 && rows % 32 != 0 && rows % 32 <= 16) ? 16 : 32;
+}
+// A CTA's rows [row0, row0 + rows) of an operand block (or panel), a multiple of 8: the
+// block's tiles of 1 << tile_log2 rows (the last, tile `last`, of tail rows) start at dst_off;
+// the rows' exponents go to exps[exp0..].
+struct DOzPack {
+  int64_t dst_off;
+  int seg0, nseg, rows, row0, k, nks, exp0, tile_log2, last, tail;
+};
+constexpr int kOzPackRows = 128, kOzPackElems = 4096;
+// CTA rows [row, row + n): element (i, k) at src_off + i rstride + k kstride; kstride 0: the
+// source is tiled (DOzTiled).
+struct DOzSeg {
+  int64_t src_off;
+  int row, n, rstride, kstride;
+};
+// One (A, B) pair: byte offsets of the blocks' (or stacked panels') tile grids, their
+// exponents, K slices, and a stacked panel's first row_map entry.
+struct DOzPair {
+  int64_t a_pk, b_pk;
+  int a_exp, b_exp, nks, map;
+};
+// A tiled FP64 intermediate (the result of stacked panels, read once by the next packing):
+// per panel the GEMM's 128 x 32 output tiles as they are, tile (tm, tn) at base + (tm ntn +
+// tn) 4096, so that both sides move whole sectors whatever the block dimensions.  row0: the
+// panel row at which a block starts.
+struct DOzTiled {
+  int64_t base;
+  int ntn, row0;
+};
+struct OzGemmArgs {
+  const uint8_t *Apk, *Bpk;
+  const int *Aexp, *Bexp;
+  const int *flag_a, *flag_b;  // equal to seq_a / seq_b: the operand's last packing flagged it
+  int seq_a, seq_b;
+  const DTile* tiles;
+  const int* cta_ptr;  // tiles [cta_ptr[c], cta_ptr[c + 1]) of CTA c
+  int nctas;
+  const DGemmTask* tasks;
+  const DOzPair* pairs;
+  const DOzTiled* pairs_tiled;  // per pair: the tiled result's panel (tiled_out), the row
+                                // operand's block in a tiled intermediate (tiled_in)
+  int tiled_out, tiled_in;
+  const int64_t* row_map;  // stacked panels: (task << 32 | row) per panel row, -1 padding
+  double alpha;
+  double *C, *partial;
+  int swap;    // tiles hold the transposed result: rows are the task's columns
+  int assign;  // C = instead of C +=
+  int* err;
+  uint64_t timeout_ns;
+  // the FP64 operands (plain path of flagged operands)
+  const double *A, *B;
+  const DGemmPair* fpairs;
+  int ta, tb;
+};
+void launch_gemm_oz(const OzGemmArgs& a, cudaStream_t st);
+void launch_oz_reduce(const DReduce* red, int nred, const OzGemmArgs& a, cudaStream_t st);
+void launch_oz_pack(const DOzPack* packs, int npacks, const DOzSeg* segs, const double* src, uint8_t* dst, int* exps,
+                    int* flag, int seq, cudaStream_t st);
 
 void launch_gemm_f64(int transa, int transb, double alpha, const double* A, const double* B, double* C,
                      const DTile* tiles, int ntiles, const DGemmTask* tasks, const DGemmPair* pairs,

@@ -30,13 +30,14 @@
 //                   accumulator into FP64 registers, then release it ("acc_empty"); at
 //                   the end write FP64 C (+=), an FP64 split-K partial, or the packed A
 //                   tiles of the next GEMM (stage-1 output).
-// Every wait is bounded by a global-timer deadline; a timeout sets a shared abort
+// Every wait is bounded by a deadline in SM clocks; a timeout sets a shared abort
 // flag that ends all roles and the device error flag the host checks.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
 #include "kernels.hpp"
+#include "tc.hpp"
 
 namespace mpsxx {
 
@@ -77,10 +78,6 @@ __device__ __forceinline__ uint32_t core_off(int row, int k) {
   return (uint32_t)(((row >> 3) * (BK / 4) + (k >> 2)) * 128 + (row & 7) * 16 + (k & 3) * 4);
 }
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
 __device__ __forceinline__ uint32_t tf32_rna(float x) {
   uint32_t r;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
@@ -92,15 +89,6 @@ __device__ __forceinline__ void split2(double v, uint32_t& h, uint32_t& l) {
   l = tf32_rna(static_cast<float>(v - static_cast<double>(__uint_as_float(h))));
 }
 
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
-  d |= (uint64_t)1 << 46;
-  return d;
-}
-
 __host__ __device__ constexpr uint32_t tf32_idesc(int m, int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
@@ -110,92 +98,6 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a, uint64_t b
       "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "l"(a), "l"(b), "r"(idesc), "r"(acc));
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t mbar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(done)
-      : "r"(mbar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-// bounded wait; false on timeout (the deadline is checked on entry too, so a limit
-// already past always ends the kernel) or when another role aborted
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, uint64_t deadline,
-                                          volatile int* abort_flag) {
-  if (global_ns() > deadline) {
-    *abort_flag = 1;
-    return false;
-  }
-  while (!mbar_try(mbar, parity)) {
-    if (*abort_flag) return false;
-    if (global_ns() > deadline) {
-      *abort_flag = 1;
-      return false;
-    }
-  }
-  return true;
-}
-
-// bounded wait that ignores the abort flag: draining the kernel's own asynchronous
-// work (bulk copies, MMAs) before it frees tensor memory and exits
-__device__ __forceinline__ void mbar_drain(uint32_t mbar, uint32_t parity, uint64_t deadline) {
-  while (!mbar_try(mbar, parity) && global_ns() <= deadline) {
-  }
-}
-constexpr uint64_t DRAIN_NS = 1000000000ull;  // 1 s
-
-__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t mbar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-      "l"(src), "r"(bytes), "r"(mbar)
-      : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
-  uint32_t r[8];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 // FP32 values at base (n16 x 16 bytes) -> hi = tf32(x) in place, lo = tf32(x - hi) at
@@ -262,7 +164,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_slot;
-  const uint64_t deadline = global_ns() + timeout_ns;
+  const uint64_t deadline = deadline_in(timeout_ns);
   const bool a_single = single & kSingleA, b_single = single & kSingleB;
   const int conv = single & (kSingleA | kSingleB);
   const uint32_t a_bytes = a_single ? A1_BYTES : A_BYTES;  // A tile in global memory
@@ -309,7 +211,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       // every bulk copy issued lands before the kernel exits (after an abort the
       // consumers no longer wait for them): the last STAGES slices' phases
-      const uint64_t dl = global_ns() + DRAIN_NS;
+      const uint64_t dl = deadline_in(DRAIN_NS);
       for (int k = slice - STAGES < 0 ? 0 : slice - STAGES; k < slice; ++k)
         mbar_drain(smem_u32(&full_bar[k % STAGES]), (uint32_t)(k / STAGES) & 1u, dl);
     }
@@ -388,7 +290,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       // every MMA issued has completed before tensor memory is freed
       mma_commit(smem_u32(&drain_bar));
-      mbar_drain(smem_u32(&drain_bar), 0u, global_ns() + DRAIN_NS);
+      mbar_drain(smem_u32(&drain_bar), 0u, deadline_in(DRAIN_NS));
     }
   } else if (warp == 2 || warp == 3) {
     // ---------------- converter (FP32 A and/or B tiles) ----------------
@@ -580,7 +482,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0 && abort_flag) atomicExch(err, 1);
+  if (threadIdx.x == 0 && abort_flag) report_timeout(err);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");

@@ -76,6 +76,7 @@ void accumulate_into(Context& ctx, double alpha, const DTensor& x, std::unique_p
   DevArray<DCopy> dcp;
   dcp.upload(cp, ctx.stream);
   launch_copy(dcp.get(), static_cast<int>(cp.size()), x.d, y->d, 1, ctx.stream);
+  y->data_version = next_data_version();  // packed copies of the old data are stale
   ctx.kernel_launches += 1;
 }
 

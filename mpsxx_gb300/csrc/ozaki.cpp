@@ -1,0 +1,319 @@
+// Host side of the FP64 GEMM on the tensor cores (kernels_oz.cu): packed layouts, stacked
+// panels, tiles and launches of a GemmPlan.
+#include <algorithm>
+#include <map>
+#include <set>
+
+#include "engine.hpp"
+
+namespace mpsxx {
+
+namespace {
+
+// A block as a GEMM operand: element (row, k) at row * rstride + k * kstride.
+struct View {
+  int rows = 0, k = 0, rstride = 0, kstride = 0;
+};
+
+int slices(int k) { return (k + kOzTileK - 1) / kOzTileK; }
+
+// The packs of rows [0, rows) of a block or panel whose tiles start at o.bytes, and their
+// room: CTAs of as many rows as fit the pack kernel's registers (row operands: within one
+// 128-row tile, column operands: across 32-row tiles).  segs_of(lo, hi) appends the segments
+// of rows [lo, hi).
+template <class F>
+void pack_rows(OzOperand& o, int rows, int k, bool row_operand, F segs_of) {
+  const int nks = slices(k), log2 = row_operand ? 7 : 5, tile = 1 << log2, last = (rows - 1) / tile;
+  const int tail = row_operand ? oz_tile_rows(rows, last) : oz_tail_cols(rows, last);
+  const int most = std::min(kOzPackRows, std::max(8, kOzPackElems / (nks * kOzTileK) / 8 * 8));
+  for (int r0 = 0; r0 < rows;) {
+    const int end = row_operand ? std::min(rows, (r0 / tile + 1) * tile) : rows;
+    const int parts = (end - r0 + most - 1) / most;
+    const int n = std::min(most, ((end - r0 + parts - 1) / parts + 7) / 8 * 8);
+    DOzPack pk;
+    pk.dst_off = o.bytes;
+    pk.seg0 = static_cast<int>(o.h_segs.size());
+    segs_of(r0, std::min(r0 + n, rows));
+    pk.nseg = static_cast<int>(o.h_segs.size()) - pk.seg0;
+    pk.rows = n;
+    pk.row0 = r0;
+    pk.k = k;
+    pk.nks = nks;
+    pk.exp0 = o.rows + r0;
+    pk.tile_log2 = log2;
+    pk.last = last;
+    pk.tail = tail;
+    o.h_packs.push_back(pk);
+    r0 += n;
+  }
+  o.rows += last * tile + tail;
+  o.bytes += (int64_t(last) * tile + tail) * nks * (kOzDigits * kOzTileK * 2);
+}
+
+// Every used block by itself.  tiled: the blocks' places in a tiled source.
+void pack_blocks(OzOperand& o, const Tensor& t, const std::vector<View>& view, bool row_operand,
+                 const std::vector<DOzTiled>* tiled = nullptr) {
+  o.base.assign(view.size(), -1);
+  o.exp0.assign(view.size(), 0);
+  o.nks.assign(view.size(), 0);
+  for (size_t s = 0; s < view.size(); ++s) {
+    const View& v = view[s];
+    if (v.rows <= 0 || v.k <= 0) continue;
+    o.base[s] = o.bytes;
+    o.exp0[s] = o.rows;
+    o.nks[s] = slices(v.k);
+    pack_rows(o, v.rows, v.k, row_operand, [&](int lo, int hi) {
+      if (tiled == nullptr) {
+        o.h_segs.push_back(DOzSeg{t.offsets[s] + int64_t(lo) * v.rstride, 0, hi - lo, v.rstride, v.kstride});
+        return;
+      }
+      const DOzTiled& p = (*tiled)[s];
+      for (int r = lo; r < hi;) {  // runs of rows inside one tile row
+        const int at = p.row0 + r, in = at % kOzTileM, run = std::min(hi - r, kOzTileM - in);
+        o.h_segs.push_back(DOzSeg{p.base + int64_t(at / kOzTileM) * p.ntn * (kOzTileM * kOzTileN) +
+                                      int64_t(in) * kOzTileN,
+                                  r - lo, run, kOzTileN, 0});
+        r += run;
+      }
+    });
+  }
+}
+
+void upload_operand(Context& ctx, OzOperand& o) {
+  o.packs.upload(o.h_packs, ctx.stream);
+  o.segs.upload(o.h_segs, ctx.stream);
+}
+
+}  // namespace
+
+void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a, const Tensor& b, bool tiled_out,
+                   const OzGemm* from, const GemmPlan* from_plan) {
+  // operand blocks as rows x K
+  std::vector<View> va(a.tags.size()), vb(b.tags.size());
+  std::set<int32_t> used_a, used_b;
+  bool single = true;
+  for (const DGemmTask& t : g.h_tasks) {
+    single = single && t.p1 - t.p0 == 1;
+    for (int p = t.p0; p < t.p1; ++p) {
+      const DGemmPair& pr = g.h_pairs[p];
+      va[g.pair_a_slot[p]] = g.ta == kNoTrans ? View{t.m, pr.k, pr.lda, 1} : View{t.m, pr.k, 1, pr.lda};
+      vb[g.pair_b_slot[p]] = g.tb == kNoTrans ? View{t.n, pr.k, 1, pr.ldb} : View{t.n, pr.k, pr.ldb, 1};
+      if (single) {
+        used_a.insert(g.pair_a_slot[p]);
+        used_b.insert(g.pair_b_slot[p]);
+      }
+    }
+  }
+  og.stacked = single;
+  og.swap = single && from == nullptr && !tiled_out && used_a.size() < used_b.size();
+  og.tiled_out = tiled_out;
+  og.tiled_in = from != nullptr;
+  if (tiled_out && !single) throw Error(kInternal, "sliced gemm plan: a tiled result needs stacked panels");
+  std::vector<DOzTiled> place, pairs_tiled;  // by block slot of a; by pair
+  if (from != nullptr) {
+    place.assign(a.tags.size(), DOzTiled{0, 0, 0});
+    for (size_t ti = 0; ti < from_plan->task_ctag.size(); ++ti) {
+      const int32_t s = a.find(from_plan->task_ctag[ti]);
+      if (s < 0) throw Error(kInternal, "sliced gemm plan: tiled block missing");
+      place[s] = from->task_place[ti];
+    }
+    for (size_t p = 0; p < g.h_pairs.size(); ++p) {
+      pairs_tiled.push_back(place[g.pair_a_slot[p]]);
+      if (pairs_tiled.back().ntn == 0) throw Error(kInternal, "sliced gemm plan: tiled block without a place");
+    }
+    single = false;  // block by block
+    og.stacked = false;
+  }
+  const Tensor& ra = og.swap ? b : a;
+  const Tensor& rb = og.swap ? a : b;
+  const std::vector<View>& vra = og.swap ? vb : va;
+  const std::vector<View>& vrb = og.swap ? va : vb;
+  auto slot_a = [&](int p) { return og.swap ? g.pair_b_slot[p] : g.pair_a_slot[p]; };
+  auto slot_b = [&](int p) { return og.swap ? g.pair_a_slot[p] : g.pair_b_slot[p]; };
+  pack_blocks(og.b, rb, vrb, false);
+  std::vector<DOzPair> pairs;
+  std::vector<int64_t> row_map;
+  if (!single) {
+    pack_blocks(og.a, ra, vra, true, from != nullptr ? &place : nullptr);
+    pairs.resize(g.h_pairs.size());
+    for (size_t p = 0; p < pairs.size(); ++p) {
+      const int32_t as = slot_a(static_cast<int>(p)), bs = slot_b(static_cast<int>(p));
+      if (og.a.nks[as] != og.b.nks[bs]) throw Error(kInternal, "sliced gemm plan: operand packing mismatch");
+      pairs[p] = DOzPair{og.a.base[as], og.b.base[bs], og.a.exp0[as], og.b.exp0[bs], og.a.nks[as], 0};
+    }
+    make_tiles(g, kOzTileM, kOzTileN, og.h_tiles, og.h_reduce, og.nslots, kOzTargetTiles);
+    for (DTile& t : og.h_tiles) {
+      t.h64 = oz_tile_rows(g.h_tasks[t.task].m, t.tm);
+      t.nt = oz_tail_cols(g.h_tasks[t.task].n, t.tn);
+    }
+  } else {
+    std::map<int32_t, std::vector<int>> panels;  // column operand block -> tasks in order
+    for (size_t ti = 0; ti < g.h_tasks.size(); ++ti)
+      panels[slot_b(g.h_tasks[ti].p0)].push_back(static_cast<int>(ti));
+    OzOperand& o = og.a;
+    for (const auto& kv : panels) {
+      const View& vc = vrb[kv.first];
+      int64_t rows = 0;
+      for (int ti : kv.second) rows += vra[slot_a(g.h_tasks[ti].p0)].rows;
+      if (rows > (int64_t(1) << 30) || row_map.size() + rows > 0x7fffff00)
+        throw Error(kInternal, "sliced gemm plan: panel too tall");
+      const int R = static_cast<int>(rows), panel = static_cast<int>(pairs.size());
+      pairs.push_back(DOzPair{o.bytes, og.b.base[kv.first], o.rows, og.b.exp0[kv.first], slices(vc.k),
+                              static_cast<int>(row_map.size())});
+      const int ntn = (vc.rows + kOzTileN - 1) / kOzTileN;
+      if (tiled_out) {
+        og.task_place.resize(g.h_tasks.size());
+        int at = 0;
+        for (int ti : kv.second) {
+          og.task_place[ti] = DOzTiled{og.tiled_elems, ntn, at};
+          at += vra[slot_a(g.h_tasks[ti].p0)].rows;
+        }
+        pairs_tiled.push_back(DOzTiled{og.tiled_elems, ntn, 0});
+        og.tiled_elems += int64_t((R + kOzTileM - 1) / kOzTileM) * ntn * (kOzTileM * kOzTileN);
+      }
+      for (int ti : kv.second)
+        for (int r = 0; r < vra[slot_a(g.h_tasks[ti].p0)].rows; ++r)
+          row_map.push_back((int64_t(ti) << 32) | int64_t(r));
+      for (int tr = 0; tr * kOzTileM < R; ++tr) {
+        const int rt = oz_tile_rows(R, tr);
+        for (int tn = 0; tn < ntn; ++tn)
+          og.h_tiles.push_back(DTile{kv.second[0], tr, tn, panel, panel + 1, -1, rt, oz_tail_cols(vc.rows, tn)});
+        if (tr * kOzTileM + rt > R)  // padding rows of the last tile
+          row_map.insert(row_map.end(), tr * kOzTileM + rt - R, -1);
+      }
+      size_t j0 = 0;  // first task that reaches the next rows, and its first panel row
+      int first = 0;
+      pack_rows(o, R, vc.k, true, [&](int lo, int hi) {
+        while (j0 < kv.second.size() && first + vra[slot_a(g.h_tasks[kv.second[j0]].p0)].rows <= lo)
+          first += vra[slot_a(g.h_tasks[kv.second[j0++]].p0)].rows;
+        int at = first;
+        for (size_t j = j0; j < kv.second.size() && at < hi; ++j) {
+          const int32_t as = slot_a(g.h_tasks[kv.second[j]].p0);
+          const View& v = vra[as];
+          if (v.k != vc.k) throw Error(kInternal, "sliced gemm plan: panel shapes differ");
+          const int x = std::max(at, lo), y = std::min(at + v.rows, hi);
+          if (x < y)
+            o.h_segs.push_back(DOzSeg{ra.offsets[as] + int64_t(x - at) * v.rstride, x - lo, y - x, v.rstride, v.kstride});
+          at += v.rows;
+        }
+      });
+    }
+  }
+  // Tiles to CTAs, heaviest first to the least loaded one: about 8 units (100 clocks) for a
+  // K step of a 32-column tile, 6 of a 16-column one, 6 for a group's hand-over.
+  std::vector<std::pair<int64_t, int>> order(og.h_tiles.size());
+  for (size_t i = 0; i < order.size(); ++i) {
+    const DTile& t = og.h_tiles[i];
+    int64_t w = 6;
+    for (int p = t.p0; p < t.p1; ++p)
+      w += int64_t(pairs[p].nks) * (t.nt == kOzTileN ? 8 : 6) + 6 * ((pairs[p].nks + kOzGroupSteps - 1) / kOzGroupSteps);
+    order[i] = {-w, static_cast<int>(i)};
+  }
+  std::stable_sort(order.begin(), order.end());
+  int nsm = 0;
+  cuda_check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx.device), "multiprocessor count");
+  const int ncta = std::min<int>(std::max(nsm, 1), static_cast<int>(order.size()));
+  std::vector<std::vector<int>> list(ncta);
+  std::vector<std::pair<int64_t, int>> heap;  // (-load, -CTA): the least loaded on top
+  for (int c = 0; c < ncta; ++c) heap.push_back({0, -c});
+  std::make_heap(heap.begin(), heap.end());
+  for (const auto& o : order) {
+    std::pop_heap(heap.begin(), heap.end());
+    list[-heap.back().second].push_back(o.second);
+    heap.back().first += o.first;
+    std::push_heap(heap.begin(), heap.end());
+  }
+  std::vector<DTile> sorted;
+  sorted.reserve(order.size());
+  og.h_cta_ptr.assign(1, 0);
+  for (const auto& l : list) {
+    for (int i : l) sorted.push_back(og.h_tiles[i]);
+    og.h_cta_ptr.push_back(static_cast<int>(sorted.size()));
+  }
+  og.h_tiles.swap(sorted);
+  og.tiles.upload(og.h_tiles, ctx.stream);
+  og.cta_ptr.upload(og.h_cta_ptr, ctx.stream);
+  if (!pairs_tiled.empty()) og.pairs_tiled.upload(pairs_tiled, ctx.stream);
+  og.pairs.upload(pairs, ctx.stream);
+  if (og.stacked) og.row_map.upload(row_map, ctx.stream);
+  og.reduce.upload(og.h_reduce, ctx.stream);
+  upload_operand(ctx, og.a);
+  upload_operand(ctx, og.b);
+  og.built = true;
+}
+
+bool oz_wanted(const Context& ctx, double flops) {
+  return flops >= (ctx.oz_min_flops >= 0.0 ? ctx.oz_min_flops : kOzMinFlops);
+}
+
+bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs) {
+  int64_t need = 0;
+  for (OzGemm* g : gs)
+    if (!g->held()) need += g->device_bytes();
+  if (need > kOzSmallBytes) {
+    size_t free_b = 0, total_b = 0;
+    cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+    if (need > static_cast<int64_t>((free_b + block_cache_bytes()) / 2)) return false;
+  }
+  try {
+    for (OzGemm* g : gs)
+      for (OzOperand* o : {&g->a, &g->b}) {
+        const bool fresh = o->exps.p == nullptr;
+        o->buf.ensure(std::max<int64_t>(o->bytes, 16), ctx.stream);
+        o->exps.ensure(size_t(o->rows + 1) * sizeof(int), ctx.stream);
+        if (fresh) cuda_check(cudaMemsetAsync(o->exps.as<int>() + o->rows, 0, sizeof(int), ctx.stream), "flag zero");
+      }
+  } catch (const Error& e) {
+    if (e.code != kAlloc) throw;
+    for (OzGemm* g : gs) g->release();
+    return false;
+  }
+  return true;
+}
+
+void oz_pack(Context& ctx, OzOperand& o, const double* src) {
+  ++o.seq;
+  launch_oz_pack(o.packs.get(), static_cast<int>(o.h_packs.size()), o.segs.get(), src, o.buf.as<uint8_t>(),
+                 o.exps.as<int>(), o.exps.as<int>() + o.rows, o.seq, ctx.stream);
+  ctx.kernel_launches += 1;
+}
+
+void run_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, double alpha, const double* A, const double* B, double* C,
+                 bool assign) {
+  ctx.gemm_part.ensure(std::max<size_t>(og.partial_bytes(), 16), ctx.stream);
+  OzGemmArgs a{};
+  a.Apk = og.a.buf.as<uint8_t>();
+  a.Bpk = og.b.buf.as<uint8_t>();
+  a.Aexp = og.a.exps.as<int>();
+  a.Bexp = og.b.exps.as<int>();
+  a.flag_a = a.Aexp + og.a.rows;
+  a.flag_b = a.Bexp + og.b.rows;
+  a.seq_a = og.a.seq;
+  a.seq_b = og.b.seq;
+  a.tiles = og.tiles.get();
+  a.cta_ptr = og.cta_ptr.get();
+  a.nctas = static_cast<int>(og.h_cta_ptr.size()) - 1;
+  a.pairs_tiled = og.pairs_tiled.get();
+  a.tiled_out = og.tiled_out;
+  a.tiled_in = og.tiled_in;
+  a.tasks = g.dtasks.get();
+  a.pairs = og.pairs.get();
+  a.row_map = og.stacked ? og.row_map.get() : nullptr;
+  a.alpha = alpha;
+  a.C = C;
+  a.partial = ctx.gemm_part.as<double>();
+  a.swap = og.swap;
+  a.assign = assign;
+  a.err = device_err_flag(ctx);
+  a.timeout_ns = ctx.device_timeout_ns;
+  a.A = A;
+  a.B = B;
+  a.fpairs = g.pairs.get();
+  a.ta = g.ta == kTrans;
+  a.tb = g.tb == kTrans;
+  launch_gemm_oz(a, ctx.stream);
+  launch_oz_reduce(og.reduce.get(), static_cast<int>(og.h_reduce.size()), a, ctx.stream);
+  ctx.kernel_launches += 1 + !og.h_reduce.empty();
+}
+
+}  // namespace mpsxx
