@@ -306,6 +306,7 @@ Context::Context(int dev, cudaStream_t st) : device(dev) {
   }
   solver_check(cusolverDnCreate(&solver), "cusolverDnCreate");
   solver_check(cusolverDnSetStream(solver, stream), "cusolverDnSetStream");
+  cuda_check(cudaEventCreateWithFlags(&dv_done, cudaEventDisableTiming), "davidson event");
   block_cache().register_stream(stream);
 }
 
@@ -317,7 +318,8 @@ Context::~Context() {
   merge_plans.clear();
   renorm_plans.clear();
   release_err_flag(*this);
-  for (DevBuf* b : {&scr1, &scr2, &work, &partial, &scalars, &svd_work, &svd_mats, &gemm_part, &svd_gram, &svd_gram_work, &svd_ptrs})
+  for (DevBuf* b : {&scr1, &scr2, &work, &partial, &scalars, &svd_work, &svd_mats, &gemm_part, &svd_gram, &svd_gram_work, &svd_ptrs,
+                    &dv_sums})
     b->release();
   forget_stream_uploads(stream);
   for (auto& l : svd_lanes) {
@@ -331,6 +333,7 @@ Context::~Context() {
     cudaStreamDestroy(l->stream);
   }
   if (svd_ready) cudaEventDestroy(svd_ready);
+  if (dv_done) cudaEventDestroy(dv_done);
   block_cache().unregister_stream(stream);
   if (solver) cusolverDnDestroy(solver);
   if (solver_params) cusolverDnDestroyParams(solver_params);
@@ -1485,9 +1488,9 @@ void apply_sigma(Context& ctx, SigmaPlan& p, const DTensor& L, const DTensor& R,
   sigma_run(ctx, p, L, R, psi, sigma, precision);
 }
 
-// Error flags of the tensor-core kernels: one int per context in mapped host memory, which a
-// kernel writes only when it gives up, so that the host reads it without a copy.  The page
-// is never freed; slots are handed out again.
+// Mapped host memory of a context, 512 bytes: the error flag of the tensor-core kernels, which
+// a kernel writes only when it gives up, so that the host reads it without a copy, and the
+// sums that the Davidson loop reads.  The page is never freed; slots are handed out again.
 namespace {
 class ErrSlots {
  public:
@@ -1495,10 +1498,10 @@ class ErrSlots {
     std::lock_guard<std::mutex> lk(mu_);
     if (free_.empty()) {
       int* page = nullptr;
-      cuda_check(cudaHostAlloc(reinterpret_cast<void**>(&page), kSlots * sizeof(int),
+      cuda_check(cudaHostAlloc(reinterpret_cast<void**>(&page), kSlots * kBytes,
                                cudaHostAllocPortable | cudaHostAllocMapped),
                  "error flag page");
-      for (int i = 0; i < kSlots; ++i) free_.push_back(page + i);
+      for (int i = 0; i < kSlots; ++i) free_.push_back(page + i * (kBytes / sizeof(int)));
     }
     int* s = free_.back();
     free_.pop_back();
@@ -1511,7 +1514,7 @@ class ErrSlots {
   }
 
  private:
-  static constexpr int kSlots = 1024;
+  static constexpr int kSlots = 128, kBytes = 512;
   std::mutex mu_;
   std::vector<int*> free_;
 };
@@ -1527,6 +1530,14 @@ int* device_err_flag(Context& ctx) {
     cuda_check(cudaHostGetDevicePointer(reinterpret_cast<void**>(&ctx.err_dev), ctx.err_host, 0), "error flag pointer");
   }
   return ctx.err_dev;
+}
+
+// 32 mapped host doubles of the context (the line after its error flag): *host as the host
+// sees them; returned as the device does.
+double* device_host_sums(Context& ctx, double** host) {
+  int* dev = device_err_flag(ctx);
+  *host = reinterpret_cast<double*>(ctx.err_host) + 8;
+  return reinterpret_cast<double*>(dev) + 8;
 }
 
 void release_err_flag(Context& ctx) {
@@ -2348,8 +2359,18 @@ static double davidson_run(Context& ctx, const DTensor& L, const DTensor& R, con
   ctx.partial.ensure(size_t(nblk) * 100 * sizeof(double), ctx.stream);
   ctx.scalars.ensure(256 * sizeof(double), ctx.stream);
   double* part = ctx.partial.as<double>();
-  double* sc = ctx.scalars.as<double>();  // [0..99] dots, [100] norm, [101] dot, [128..227] rvec, [230..] roots
-  double* rvec_d = sc + 128;
+  double* sc = ctx.scalars.as<double>();  // [230..] roots
+  // sums of the fused vector kernels: [row 0] subspace row, [1] residual, [2], [3] projections
+  const bool fresh = ctx.dv_sums.p == nullptr;
+  ctx.dv_sums.ensure((64 + dv_partial_doubles()) * sizeof(double), st);
+  double* ds = ctx.dv_sums.as<double>();
+  if (fresh) cuda_check(cudaMemsetAsync(ds, 0, sizeof(double), st), "ticket zero");
+  double *hrow, *hres;  // mapped host copies of rows 0 and 1
+  double* drow = device_host_sums(ctx, &hrow);
+  hres = hrow + 16;
+  auto sums = [&](int row, double* host) {
+    return DvReduce{ds + 64, ds + 1 + 12 * row, host, reinterpret_cast<unsigned*>(ds)};
+  };
 
   PhaseTimer trest(ctx, kPhDavidsonRest);
   // Lower roots (multi-root, src/diagonalize.hpp:200-277): with s_j = <S_j|c> and
@@ -2372,8 +2393,7 @@ static double davidson_run(Context& ctx, const DTensor& L, const DTensor& R, con
   };
   auto sigma_of = [&](int k, int precision) {
     PhaseTimer tm(ctx, precision == kFP64 && ctx.precision != kFP64 ? kPhSigmaFP64 : kPhSigma);
-    cuda_check(cudaMemsetAsync(sigma + k * n, 0, n * sizeof(double), st), "sigma zero");
-    sigma_run(ctx, sp, L, R, trial + k * n, sigma + k * n, precision);
+    sigma_run(ctx, sp, L, R, trial + k * n, sigma + k * n, precision);  // (zeroed with trial k)
     S.n_sigma += 1;
     if (precision == kFP64) S.n_sigma_fp64 += 1;
     tm.stop();
@@ -2395,45 +2415,70 @@ static double davidson_run(Context& ctx, const DTensor& L, const DTensor& R, con
     for (size_t j = 0; j < proj->S.size(); ++j) launch_axpy(c, proj->S[j], n, -pdots[2 * j], st);
     ctx.kernel_launches += static_cast<int64_t>(proj->S.size());
   };
-  auto normalize = [&](double* x) {
-    launch_multidot(x, 1, x, 1, n, n, sc + 100, part, nblk, st);
-    launch_scal_dev(x, n, sc + 100, 1, st);
-    ctx.kernel_launches += 3;
+  auto normalize = [&](double* x, double* zero) {
+    launch_dv_dots(x, x, 1, n, sums(0, nullptr), st);
+    launch_dv_scaled_copy(x, n, sums(0, nullptr).out, x, zero, st);
+    ctx.kernel_launches += 2;
+  };
+  auto wait = [&] {
+    cuda_check(cudaEventRecord(ctx.dv_done, st), "davidson event");
+    return ctx.dv_done;
   };
 
   launch_copy_vec(trial, wfnc.d, n, st);
   orthogonalize_roots(trial);
   double eval = 0.0;
   int niter = 0, iconv = 0;
-  std::vector<double> hdots(100), heff, rvec, rval;
+  // Ritz vectors of the last iteration: rit[i*10 + j] = component on trial i of vector j.
+  // The subspace matrix is formed in their basis (diagonal but for the new vector's row), as
+  // if the trial vectors had been rotated; the trial vectors themselves stay.
+  std::vector<double> hsub, q, rval, rit(max_ritz * max_ritz), rnew(max_ritz);
+  DvCoef coef{};
   while (iconv < 1 && niter < max_macro) {
-    normalize(trial);
+    normalize(trial, sigma);
     sigma_of(0, anchor && niter == 0 ? kFP64 : ctx.precision);
-    for (int m = 1; m <= max_ritz; ++m) {
-      launch_multidot(trial, m, sigma, m, n, n, sc, part, nblk, st);
-      ctx.kernel_launches += 2;
-      cuda_check(cudaMemcpyAsync(hdots.data(), sc, m * m * sizeof(double), cudaMemcpyDeviceToHost, st), "heff d2h");
-      ctx.sync();
-      heff.assign(m * m, 0.0);
-      for (int i = 0; i < m; ++i)
-        for (int j = 0; j <= i; ++j) {
-          const double h = hdots[i * m + j];  // trial_i . sigma_j
-          heff[i * m + j] = h;
-          heff[j * m + i] = h;
+    std::fill(rit.begin(), rit.end(), 0.0);
+    int m = 1;
+    for (; m <= max_ritz; ++m) {
+      const int k = m - 1;  // the new vector
+      launch_dv_dots(trial + k * n, sigma, m, n, sums(0, drow), st);
+      ctx.kernel_launches += 1;
+      cuda_check(cudaEventSynchronize(wait()), "subspace row");
+      hsub.assign(m * m, 0.0);
+      for (int j = 0; j < k; ++j) {
+        double h = 0.0;  // trial_k . (sigma of Ritz vector j)
+        for (int i = 0; i < k; ++i) h += rit[i * max_ritz + j] * hrow[i];
+        hsub[k * m + j] = hsub[j * m + k] = h;
+        hsub[j * m + j] = rval[j];
+      }
+      hsub[k * m + k] = hrow[k];
+      jacobi_eigh(m, hsub, rval, q);  // q[i*m + j]: component i of eigenvector j
+      rit[k * max_ritz + k] = 1.0;
+      for (int i = 0; i < m; ++i) {
+        for (int j = 0; j < m; ++j) {
+          double r = 0.0;
+          for (int l = 0; l < m; ++l) r += rit[i * max_ritz + l] * q[l * m + j];
+          rnew[j] = r;
         }
-      jacobi_eigh(m, heff, rval, rvec);  // rvec[i*m + j]: component i of eigenvector j
+        std::copy(rnew.begin(), rnew.begin() + m, rit.begin() + i * max_ritz);
+        coef.v[i] = rnew[0];
+      }
       eval = rval[0];
       S.micro += 1;
-      upload_staged(rvec_d, rvec.data(), m * m * sizeof(double), st);
-      launch_rotate(trial, m, n, n, rvec_d, m, nullptr, st);
-      launch_rotate(sigma, m, n, n, rvec_d, m, nullptr, st);
-      launch_copy_vec(errv, sigma, n, st);
-      launch_axpy(errv, trial, n, -eval, st);
-      launch_multidot(errv, 1, errv, 1, n, n, sc + 101, part, nblk, st);
-      ctx.kernel_launches += 6;
-      double rnorm = 0.0;
-      cuda_check(cudaMemcpyAsync(&rnorm, sc + 101, sizeof(double), cudaMemcpyDeviceToHost, st), "rnorm d2h");
-      ctx.sync();
+      launch_dv_residual(trial, sigma, diag.d, m, n, coef, eval, errv, sums(1, drow + 16), st);
+      const cudaEvent_t done = wait();
+      ctx.kernel_launches += 1;
+      if (m < max_ritz) {
+        // correction vector orthonormalised against the subspace: the reference projects
+        // out one trial vector at a time (src/diagonalize.hpp:425-431); here classical
+        // Gram-Schmidt is applied twice.  Queued before the residual is known: one that
+        // turns out converged has no use for it.
+        launch_dv_project(trial, m, n, errv, sums(1, nullptr).out, 0, sums(2, nullptr), st);
+        launch_dv_project(trial, m, n, errv, sums(2, nullptr).out, 1, sums(3, nullptr), st);
+        ctx.kernel_launches += 2;
+      }
+      cuda_check(cudaEventSynchronize(done), "residual");
+      const double rnorm = hres[0];
       S.rnorm = rnorm;
       if (anchor && niter == 0 && m == 1) S.rnorm_fp64 = rnorm;
       if (rnorm < tol || (rel_floor > 0.0 && rnorm < rel_floor * rel_floor * eval * eval)) {
@@ -2441,30 +2486,21 @@ static double davidson_run(Context& ctx, const DTensor& L, const DTensor& R, con
         break;
       }
       if (m < max_ritz) {
-        // correction vector orthonormalised against the subspace: the reference
-        // projects out one trial vector at a time (src/diagonalize.hpp:425-431); here
-        // classical Gram-Schmidt is applied twice, all m projections per pass in one
-        // multi-dot and one update (the same vector to rounding, 12 launches for m)
-        launch_precondition(errv, diag.d, n, eval, st);
-        normalize(errv);
-        for (int pass = 0; pass < 2; ++pass) {
-          launch_multidot(trial, m, errv, 1, n, n, sc + 104, part, nblk, st);
-          launch_project_out(errv, trial, m, n, n, sc + 104, st);
-          ctx.kernel_launches += 3;
-        }
-        normalize(errv);
-        launch_copy_vec(trial + m * n, errv, n, st);
-        ctx.kernel_launches += 2;
+        launch_dv_scaled_copy(errv, n, sums(3, nullptr).out, trial + m * n, sigma + m * n, st);
+        ctx.kernel_launches += 1;
         sigma_of(m, ctx.precision);
       }
     }
+    launch_dv_combine(trial, std::min(m, max_ritz), n, coef, trial, st);  // the Ritz vector
+    ctx.kernel_launches += 1;
     ++niter;
   }
   S.macro += niter;
   S.converged = iconv;
   launch_copy_vec(wfnc.d, trial, n, st);
   orthogonalize_roots(wfnc.d);  // multH.orthonormalize (src/diagonalize.hpp:446)
-  normalize(wfnc.d);
+  normalize(wfnc.d, nullptr);
+  wfnc.data_version = next_data_version();
   ctx.sync();
   return eval;
 }

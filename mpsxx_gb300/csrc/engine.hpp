@@ -392,6 +392,8 @@ struct Context {
   DevBuf work;       // Davidson vectors
   DevBuf partial;    // reduction partials
   DevBuf scalars;    // small device scalars
+  DevBuf dv_sums;    // Davidson: ticket, sums and partials of the fused vector kernels
+  cudaEvent_t dv_done = nullptr;
   DevBuf svd_work;   // solver workspace
   DevBuf svd_mats;   // per-block SVD matrices
   DevBuf gemm_part;  // split-K partial tiles
@@ -510,6 +512,7 @@ void compute_sigma_vector(Context& ctx, const DTensor& L, const DTensor& R, cons
 
 int* device_err_flag(Context& ctx);
 void release_err_flag(Context& ctx);
+double* device_host_sums(Context& ctx, double** host);
 void check_device_error(Context& ctx);
 
 // average device seconds of `reps` sigma applications (CUDA events on ctx.stream)

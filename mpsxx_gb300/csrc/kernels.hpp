@@ -292,9 +292,7 @@ void launch_diag(const DDiagTask* tasks, int ntasks, const DDiagPair* pairs, con
                  double* out, int max_tiles, cudaStream_t st);
 
 // Level-1 over dense vectors of length n (the block layout of a wavefunction).
-void launch_fill(double* x, int64_t n, double v, cudaStream_t st);
 void launch_scal_dev(double* x, int64_t n, const double* s, int mode, cudaStream_t st);
-void launch_axpy_dev(double* y, const double* x, int64_t n, const double* s, double sign, cudaStream_t st);
 void launch_axpy(double* y, const double* x, int64_t n, double a, cudaStream_t st);
 void launch_copy_vec(double* y, const double* x, int64_t n, cudaStream_t st);
 // y[b.off + j] = y[b.off + j] + noise * seq[j] for every block b (product and sum
@@ -304,13 +302,31 @@ void launch_noise_axpy(const DNoise* blocks, int nblocks, const double* seq, dou
 // out[i*m + j] = dot(X_i, Y_j) for i < nx, j < ny (vectors strided by `stride`)
 void launch_multidot(const double* X, int nx, const double* Y, int ny, int64_t n, int64_t stride, double* out,
                      double* partial, int nblocks, cudaStream_t st);
-// new_j = sum_i R[i*ld + j] * old_i, j < m (in place via scratch `tmp` of m*n)
-void launch_rotate(double* V, int m, int64_t n, int64_t stride, const double* R, int ldr, double* tmp,
-                   cudaStream_t st);
-// y -= sum_{i < m} c[i] X[i * stride : i * stride + n], c (m values) on the device
-void launch_project_out(double* y, const double* X, int m, int64_t n, int64_t stride, const double* c,
-                        cudaStream_t st);
-void launch_precondition(double* r, const double* diag, int64_t n, double e, cudaStream_t st);
+// Davidson vector algebra (kernels_davidson.cu).  Sums of a launch: at most kMaxDot + 2,
+// through partial (dv_partial_doubles) into out on the device and, unless null, into host
+// (mapped memory); ticket is zero between launches.
+struct DvReduce {
+  double *partial, *out, *host;
+  unsigned* ticket;
+};
+struct DvCoef {
+  double v[kMaxDot];
+};
+size_t dv_partial_doubles();
+// out[j] = x . Y_j (vectors n apart), j < m
+void launch_dv_dots(const double* x, const double* Y, int m, int64_t n, const DvReduce& rd, cudaStream_t st);
+// c = (s - e t) / (e - diag) with t = sum r_i T_i, s = sum r_i S_i; out = [|s - e t|^2, |c|^2,
+// T_i . c]
+void launch_dv_residual(const double* T, const double* S, const double* diag, int m, int64_t n, const DvCoef& r,
+                        double e, double* c, const DvReduce& rd, cudaStream_t st);
+// Gram-Schmidt pass: first: c normalised (in = launch_dv_residual's sums) and projected, out =
+// T_i . c; second: projected once more with in = those, out = |c|^2
+void launch_dv_project(const double* T, int m, int64_t n, double* c, const double* in, int second, const DvReduce& rd,
+                       cudaStream_t st);
+// t = x / sqrt(in[0]) (t may be x), z = 0 (z may be null)
+void launch_dv_scaled_copy(const double* x, int64_t n, const double* in, double* t, double* z, cudaStream_t st);
+// out = sum r_i T_i (out may be T_0)
+void launch_dv_combine(const double* T, int m, int64_t n, const DvCoef& r, double* out, cudaStream_t st);
 void launch_scale_blocks_rows(double* data, const int64_t* off, const int* rows, const int* cols,
                               const int64_t* s_off, int nb, const double* s, cudaStream_t st);
 void launch_scale_blocks_cols(double* data, const int64_t* off, const int* rows, const int* cols,

@@ -298,22 +298,11 @@ __global__ void __launch_bounds__(256) diag_kernel(const DDiagTask* __restrict__
   }
 }
 
-__global__ void fill_kernel(double* x, int64_t n, double v) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    x[i] = v;
-}
-
 // mode 0: x *= s[0]; mode 1: x *= 1/sqrt(s[0]) (s holds a squared norm)
 __global__ void scal_dev_kernel(double* x, int64_t n, const double* s, int mode) {
   const double f = mode == 0 ? s[0] : 1.0 / sqrt(s[0]);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     x[i] *= f;
-}
-
-__global__ void axpy_dev_kernel(double* y, const double* x, int64_t n, const double* s, double sign) {
-  const double a = sign * s[0];
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = fma(a, x[i], y[i]);
 }
 
 __global__ void axpy_kernel(double* y, const double* x, int64_t n, double a) {
@@ -385,49 +374,6 @@ __global__ void multidot_final_kernel(const double* __restrict__ partial, int nb
   double v = 0.0;
   for (int b = 0; b < nblocks; ++b) v += partial[b * (kMaxDot * kMaxDot) + q];
   out[q] = v;
-}
-
-// y -= sum_{i < m} c[i] X[:, i] (X's vectors stride apart; c on the device).
-__global__ void project_out_kernel(double* __restrict__ y, const double* __restrict__ X, int m, int64_t n,
-                                   int64_t stride, const double* __restrict__ c) {
-  double cc[kMaxDot];
-#pragma unroll
-  for (int i = 0; i < kMaxDot; ++i) cc[i] = i < m ? c[i] : 0.0;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-    double v = y[e];
-#pragma unroll
-    for (int i = 0; i < kMaxDot; ++i)
-      if (i < m) v = fma(-cc[i], X[i * stride + e], v);
-    y[e] = v;
-  }
-}
-
-// V[:, j] = sum_i V[:, i] R[i, j] for j < m, in place per element (loops unrolled to
-// kMaxDot so that the element's m values stay in registers).
-__global__ void rotate_kernel(double* V, int m, int64_t n, int64_t stride, const double* __restrict__ R, int ldr) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-    double old[kMaxDot];
-#pragma unroll
-    for (int i = 0; i < kMaxDot; ++i) old[i] = i < m ? V[i * stride + e] : 0.0;
-#pragma unroll
-    for (int j = 0; j < kMaxDot; ++j) {
-      if (j < m) {
-        double v = 0.0;
-#pragma unroll
-        for (int i = 0; i < kMaxDot; ++i)
-          if (i < m) v = fma(R[i * ldr + j], old[i], v);
-        V[j * stride + e] = v;
-      }
-    }
-  }
-}
-
-__global__ void precondition_kernel(double* r, const double* __restrict__ diag, int64_t n, double e) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double denm = e - diag[i];
-    if (fabs(denm) < 1.0e-8) denm = 1.0e-8;
-    r[i] /= denm;
-  }
 }
 
 __global__ void scale_rows_kernel(double* data, const int64_t* off, const int* rows, const int* cols,
@@ -517,19 +463,9 @@ void launch_diag(const DDiagTask* tasks, int ntasks, const DDiagPair* pairs, con
   diag_kernel<<<dim3(ntasks, max_tiles), 256, 0, st>>>(tasks, pairs, L, R, out);
 }
 
-void launch_fill(double* x, int64_t n, double v, cudaStream_t st) {
-  if (n <= 0) return;
-  fill_kernel<<<grid_for(n), 256, 0, st>>>(x, n, v);
-}
-
 void launch_scal_dev(double* x, int64_t n, const double* s, int mode, cudaStream_t st) {
   if (n <= 0) return;
   scal_dev_kernel<<<grid_for(n), 256, 0, st>>>(x, n, s, mode);
-}
-
-void launch_axpy_dev(double* y, const double* x, int64_t n, const double* s, double sign, cudaStream_t st) {
-  if (n <= 0) return;
-  axpy_dev_kernel<<<grid_for(n), 256, 0, st>>>(y, x, n, s, sign);
 }
 
 void launch_axpy(double* y, const double* x, int64_t n, double a, cudaStream_t st) {
@@ -549,7 +485,7 @@ void launch_copy_vec(double* y, const double* x, int64_t n, cudaStream_t st) {
 }
 
 int multidot_blocks(int64_t n) {
-  int64_t b = (n + 2047) / 2048;
+  int64_t b = (n + 255) / 256;
   if (b > kMultidotMaxBlocks) b = kMultidotMaxBlocks;
   if (b < 1) b = 1;
   return static_cast<int>(b);
@@ -559,24 +495,6 @@ void launch_multidot(const double* X, int nx, const double* Y, int ny, int64_t n
                      double* partial, int nblocks, cudaStream_t st) {
   multidot_partial_kernel<<<nblocks, 256, 0, st>>>(X, nx, Y, ny, n, stride, partial);
   multidot_final_kernel<<<1, 128, 0, st>>>(partial, nblocks, nx * ny, out);
-}
-
-void launch_rotate(double* V, int m, int64_t n, int64_t stride, const double* R, int ldr, double* tmp,
-                   cudaStream_t st) {
-  (void)tmp;
-  if (n <= 0) return;
-  rotate_kernel<<<grid_for(n), 256, 0, st>>>(V, m, n, stride, R, ldr);
-}
-
-void launch_project_out(double* y, const double* X, int m, int64_t n, int64_t stride, const double* c,
-                        cudaStream_t st) {
-  if (n <= 0 || m <= 0) return;
-  project_out_kernel<<<grid_for(n), 256, 0, st>>>(y, X, m, n, stride, c);
-}
-
-void launch_precondition(double* r, const double* diag, int64_t n, double e, cudaStream_t st) {
-  if (n <= 0) return;
-  precondition_kernel<<<grid_for(n), 256, 0, st>>>(r, diag, n, e);
 }
 
 void launch_scale_blocks_rows(double* data, const int64_t* off, const int* rows, const int* cols,
