@@ -277,6 +277,7 @@ template struct DevArray<DGemmTask>;
 template struct DevArray<DGemmPair>;
 template struct DevArray<DDiagTask>;
 template struct DevArray<DDiagPair>;
+template struct DevArray<DDiagTile>;
 template struct DevArray<DCopy>;
 template struct DevArray<DScatterDst>;
 template struct DevArray<DScatterSrc>;
@@ -1635,8 +1636,20 @@ DiagPlan& diag_plan(Context& ctx, const Tensor& L, const Tensor& R, const Tensor
     p->h_tasks.push_back(t);
     p->ref.push_back({diag.tags[b], std::move(refp)});
   }
-  for (const DDiagTask& t : p->h_tasks)
-    p->max_tiles = std::max(p->max_tiles, ((t.m + 31) / 32) * ((t.n + 31) / 32));
+  // longest pair lists first
+  std::vector<DDiagTile> tiles;
+  for (size_t i = 0; i < p->h_tasks.size(); ++i) {
+    const DDiagTask& t = p->h_tasks[i];
+    int log2w = 0;
+    while (log2w < 5 && (1 << log2w) < t.n) ++log2w;
+    for (int a = 0; a < t.m; a += diag_rows(log2w))
+      for (int b = 0; b < t.n; b += 1 << log2w) tiles.push_back(DDiagTile{static_cast<int>(i), a, b, log2w});
+  }
+  std::stable_sort(tiles.begin(), tiles.end(), [&](const DDiagTile& x, const DDiagTile& y) {
+    return p->h_tasks[x.task].p1 - p->h_tasks[x.task].p0 > p->h_tasks[y.task].p1 - p->h_tasks[y.task].p0;
+  });
+  p->ntiles = static_cast<int>(tiles.size());
+  p->tiles.upload(tiles, ctx.stream);
   p->tasks.upload(p->h_tasks, ctx.stream);
   p->pairs.upload(p->h_pairs, ctx.stream);
   return insert_plan(ctx, ctx.diag_plans, key, std::move(p));
@@ -1644,8 +1657,7 @@ DiagPlan& diag_plan(Context& ctx, const Tensor& L, const Tensor& R, const Tensor
 
 void compute_diagonal_elements(Context& ctx, const DTensor& L, const DTensor& R, DTensor& diag) {
   DiagPlan& p = diag_plan(ctx, L, R, diag);
-  launch_diag(p.tasks.get(), static_cast<int>(p.h_tasks.size()), p.pairs.get(), L.d, R.d, diag.d, p.max_tiles,
-              ctx.stream);
+  launch_diag(p.tiles.get(), p.ntiles, p.tasks.get(), p.pairs.get(), L.d, R.d, diag.d, ctx.stream);
   ctx.kernel_launches += 1;
 }
 
@@ -1906,11 +1918,52 @@ static std::unique_ptr<MergePlan> build_merge_plan(Context& ctx, bool forward, c
         hs[fill[ent_col[e]]++] = DScatterSrc{opr.offsets[ob], sld, ent_st[e], ent_coef[e]};
     }
   }
+  // Sub-blocks that nothing contributes to: records without sources, so that the records
+  // tile every result block and the kernel writes all of it (no zeroing before)
+  std::vector<int32_t> pos_b(mb.merged_of.size()), pos_k(mk.merged_of.size());  // place among a sector's members
+  for (const auto& v : mb.members)
+    for (size_t i = 0; i < v.size(); ++i) pos_b[v[i]] = static_cast<int32_t>(i);
+  for (const auto& v : mk.members)
+    for (size_t i = 0; i < v.size(); ++i) pos_k[v[i]] = static_cast<int32_t>(i);
+  std::vector<int64_t> cover0(out->tags.size() + 1, 0);
+  std::vector<std::array<int, 3>> bi(out->tags.size());
+  for (size_t b = 0; b < out->tags.size(); ++b) {
+    out->sh.index(out->tags[b], bi[b].data());
+    cover0[b + 1] = cover0[b] + int64_t(mb.members[bi[b][0]].size()) * mk.members[bi[b][2]].size();
+  }
+  std::vector<char> covered(cover0.back(), 0);
+  for (size_t g = 0; g + 1 < group_first.size(); ++g) {
+    if (group_first[g] == group_first[g + 1]) continue;
+    const int a = oi[order[group_src[g]]][0], x = oi[order[group_src[g]]][2];
+    for (int64_t di = group_first[g]; di < group_first[g + 1]; ++di) {
+      const int st = dsts[di].col / nu, sidx = st / nt, tidx = st % nt;
+      const int ipr = forward ? a * ns + sidx : sidx * opr.sh.nsec(0) + a;
+      const int ipc = forward ? x * nt + tidx : tidx * nx + x;
+      const int32_t slot = slot_of(dsts[di].otag);
+      covered[cover0[slot] + int64_t(pos_b[ipr]) * mk.members[bi[slot][2]].size() + pos_k[ipc]] = 1;
+    }
+  }
+  std::vector<DScatterDst> all(hd);
+  for (size_t b = 0; b < out->tags.size(); ++b) {
+    const auto& rm = mb.members[bi[b][0]];
+    const auto& cm = mk.members[bi[b][2]];
+    const int dcols = out->sh.dshape[2][bi[b][2]];
+    for (size_t i = 0; i < rm.size(); ++i)
+      for (size_t j = 0; j < cm.size(); ++j) {
+        if (covered[cover0[b] + int64_t(i) * cm.size() + j]) continue;
+        DScatterDst r{};
+        r.dst_off = out->offsets[b] + int64_t(mb.offset_packed[rm[i]]) * dcols + mk.offset_packed[cm[j]];
+        r.rows = mb.d_packed[rm[i]];
+        r.cols = mk.d_packed[cm[j]];
+        r.dld = dcols;
+        if (r.rows > 0 && r.cols > 0) all.push_back(r);
+      }
+  }
   auto plan = std::make_unique<MergePlan>();
   plan->layout = static_cast<const Tensor&>(*out);
-  plan->dst.upload(hd, ctx.stream);
+  plan->dst.upload(all, ctx.stream);
   plan->src.upload(hs, ctx.stream);
-  plan->ndst = static_cast<int>(hd.size());
+  plan->ndst = static_cast<int>(all.size());
   plan->h_dst = std::move(hd);
   plan->src_entry.resize(hs.size());
   for (size_t i = 0; i < hs.size(); ++i) plan->src_entry[i] = hs[i].pad;
@@ -2012,7 +2065,7 @@ std::unique_ptr<DTensor> compute_merged_operator(Context& ctx, bool forward, con
   tplan.stop();
   PhaseTimer talloc(ctx, kPhMergeAlloc);
   out->ctx = &ctx;
-  out->alloc_device(ctx.stream, true);
+  out->alloc_device(ctx.stream, false);  // the scatter writes every element
   talloc.stop();
   PhaseTimer trun(ctx, kPhMergeRun);
   launch_scatter(plan.dst.get(), plan.ndst, plan.src.get(), opr.d, out->d, ctx.stream);

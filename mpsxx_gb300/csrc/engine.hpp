@@ -330,7 +330,8 @@ struct RenormPlan {
 };
 
 struct DiagPlan {
-  int max_tiles = 0;  // most 32 x 32 tiles of one block (the kernel's grid height)
+  int ntiles = 0;
+  DevArray<DDiagTile> tiles;
   std::vector<DDiagTask> h_tasks;
   std::vector<DDiagPair> h_pairs;
   DevArray<DDiagTask> tasks;

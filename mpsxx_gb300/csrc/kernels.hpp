@@ -63,7 +63,7 @@ struct DCopy {
   int rows, cols, dld, sld;
   double scale;
 };
-// Destination of a scatter-accumulate: sum over its sources in fixed order.
+// Destination of a scatter: the sum over its sources in fixed order (zero without sources).
 struct DScatterDst {
   int64_t dst_off;
   int rows, cols, dld, s0, s1, pad;
@@ -80,6 +80,11 @@ struct DDiagTask {
 };
 struct DDiagPair {
   int64_t l_off, r_off;
+};
+// A CTA's outputs of a diagonal task: 1 << log2w columns from b0, diag_rows rows from a0.
+__host__ __device__ constexpr int diag_rows(int log2w) { return log2w >= 2 ? 256 >> log2w : 64; }
+struct DDiagTile {
+  int task, a0, b0, log2w;
 };
 // Noise block of make_noise: y[off + j] += noise * seq[j] for j < n.
 struct DNoise {
@@ -288,8 +293,8 @@ void launch_adjoint_scatter(const DScatterDst* dsts, int ndst, const DScatterSrc
                             const double* src, double* g, cudaStream_t st);
 // G[e] = sum_{k = ptr[e]}^{ptr[e+1]-1} g[idx[k]], summed in index order.
 void launch_segment_sum(const int* ptr, const int* idx, const double* g, int ne, double* G, cudaStream_t st);
-void launch_diag(const DDiagTask* tasks, int ntasks, const DDiagPair* pairs, const double* L, const double* R,
-                 double* out, int max_tiles, cudaStream_t st);
+void launch_diag(const DDiagTile* tiles, int ntiles, const DDiagTask* tasks, const DDiagPair* pairs, const double* L,
+                 const double* R, double* out, cudaStream_t st);
 
 // Level-1 over dense vectors of length n (the block layout of a wavefunction).
 void launch_scal_dev(double* x, int64_t n, const double* s, int mode, cudaStream_t st);
