@@ -252,6 +252,8 @@ class Batch {
     int slots1 = 0;
     for (int c : members) {
       const Item& x = it_[c];
+      x.sp->s1.prepare_f64(ctx_.stream);
+      x.sp->s2.prepare_f64(ctx_.stream);
       add(x.sp->s1, x.bL64, x.off + kSlotIn * x.n, x.bScr64, t1, k1, p1, r1);
       slots += x.sp->s1.nslots;
     }

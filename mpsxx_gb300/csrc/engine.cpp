@@ -511,8 +511,7 @@ static void build_plan_impl(GemmPlan& plan, Trans ta, Trans tb, const Tensor& a,
     plan.task_ctag.push_back(t.c_tag);
     plan.c_elems += int64_t(c.m) * c.n;
   }
-  make_tiles(plan, kGemmTile, kGemmTile, plan.h_tiles, plan.h_reduce, plan.nslots, kTargetCtas);
-  tile_tc(plan, kTargetCtas);
+  plan.f64_ready = plan.tc_ready = false;
 }
 
 // Tensor-core (128 x 64) tiling of a plan's tasks with split-K chunks sized for about
@@ -555,17 +554,30 @@ void build_gemm_plan(GemmPlan& plan, Trans ta, Trans tb, const Tensor& a, const 
 }
 
 void GemmPlan::upload(cudaStream_t st) {
-  tiles.upload(h_tiles, st);
   dtasks.upload(h_tasks, st);
   pairs.upload(h_pairs, st);
+}
+
+void GemmPlan::prepare_f64(cudaStream_t st) {
+  if (f64_ready) return;
+  make_tiles(*this, kGemmTile, kGemmTile, h_tiles, h_reduce, nslots, kTargetCtas);
+  tiles.upload(h_tiles, st);
   reduce.upload(h_reduce, st);
+  f64_ready = true;
+}
+
+void GemmPlan::prepare_tc(cudaStream_t st) {
+  if (tc_ready) return;
+  tile_tc(*this, kTargetCtas);
   tiles_tc.upload(h_tiles_tc, st);
   reduce_tc.upload(h_reduce_tc, st);
+  tc_ready = true;
 }
 
 
 void GemmPlan::run(double alpha, const double* A, const double* B, double* C, double* partial,
-                   cudaStream_t st) const {
+                   cudaStream_t st) {
+  prepare_f64(st);
   if (nslots > 0 && partial == nullptr) throw Error(kInternal, "gemm plan: split-K scratch missing");
   launch_gemm_f64(ta, tb, alpha, A, B, C, tiles.get(), static_cast<int>(h_tiles.size()), dtasks.get(), pairs.get(),
                   partial, st);
@@ -573,7 +585,8 @@ void GemmPlan::run(double alpha, const double* A, const double* B, double* C, do
     launch_gemm_reduce(reduce.get(), static_cast<int>(h_reduce.size()), dtasks.get(), alpha, partial, C, st);
 }
 
-static double* gemm_scratch(Context& ctx, const GemmPlan& p) {
+static double* gemm_scratch(Context& ctx, GemmPlan& p) {
+  p.prepare_f64(ctx.stream);
   if (p.nslots == 0) return nullptr;
   ctx.gemm_part.ensure(p.partial_bytes(), ctx.stream);
   return ctx.gemm_part.as<double>();
@@ -594,7 +607,6 @@ static Tensor conj_view(const Tensor& t) {
   c.sh = t.sh.conjugate();
   c.tags = t.tags;
   c.offsets = t.offsets;
-  c.slot = t.slot;
   c.nnz = t.nnz;
   c.d = t.d;
   c.layout_id = t.layout_id;
@@ -848,6 +860,8 @@ static void build_stacked_stage1(Context& ctx, SigmaPlan& p, const Tensor& L) {
 }
 
 static void build_sigma_pk(Context& ctx, SigmaPlan& p, const Tensor& L, const Tensor& R, const Tensor& psi) {
+  p.s1.prepare_tc(ctx.stream);
+  p.s2.prepare_tc(ctx.stream);
   auto dims3 = [](const Tensor& t, int32_t b, int* d) { t.block_dims(b, d); };
   // stage 1: A = L block (dA x dA'), B^T = psi block transposed (dB' x dA'); the
   // operators as FP32 tiles (split on chip) or as hi|lo tiles
@@ -952,9 +966,10 @@ static void build_split_gemm(Context& ctx, SplitGemm& sg, const GemmPlan& g, con
 }
 
 // C += alpha * op(A) op(B) over the plan's tasks, in split TF32 (g uploaded).
-static void run_split_gemm(Context& ctx, SplitGemm& sg, const GemmPlan& g, double alpha, const double* A,
-                           const double* B, double* C) {
+static void run_split_gemm(Context& ctx, SplitGemm& sg, GemmPlan& g, double alpha, const double* A, const double* B,
+                           double* C) {
   if (g.h_tasks.empty()) return;
+  g.prepare_tc(ctx.stream);
   sg.pa.buf.ensure(std::max<int64_t>(sg.pa.bytes, 16), ctx.stream);
   sg.pb.buf.ensure(std::max<int64_t>(sg.pb.bytes, 16), ctx.stream);
   launch_pack(sg.pa.packs.get(), static_cast<int>(sg.pa.h_packs.size()), A, sg.pa.buf.as<uint8_t>(), ctx.stream);
@@ -1394,6 +1409,8 @@ static void sigma_run(Context& ctx, SigmaPlan& p, const DTensor& L, const DTenso
     ctx.scr1.ensure(std::max<int64_t>(p.scr1.nnz, 1) * sizeof(double), ctx.stream);
     double* scr = ctx.scr1.as<double>();
     if (p.scr1.nnz) cuda_check(cudaMemsetAsync(scr, 0, p.scr1.nnz * sizeof(double), ctx.stream), "scr1 zero");
+    p.s1.prepare_f64(ctx.stream);
+    p.s2.prepare_f64(ctx.stream);
     ctx.gemm_part.ensure(std::max(p.s1.partial_bytes(), p.s2.partial_bytes()), ctx.stream);
     double* part = ctx.gemm_part.as<double>();
     p.s1.run(1.0, L.d, psi, scr, part, ctx.stream);
@@ -1748,6 +1765,8 @@ std::unique_ptr<DTensor> renormalize(Context& ctx, bool forward, const DTensor& 
   } else if (oz_wanted(ctx, rp.p1.flops + rp.p2.flops) && renorm_run_oz(ctx, rp, bra, opr0, ket, sp, out->d)) {
   } else {
     zero_scr();
+    rp.p1.prepare_f64(ctx.stream);
+    rp.p2.prepare_f64(ctx.stream);
     ctx.gemm_part.ensure(std::max(rp.p1.partial_bytes(), rp.p2.partial_bytes()), ctx.stream);
     rp.p1.run(1.0, bra.d, opr0.d, sp, ctx.gemm_part.as<double>(), ctx.stream);
     rp.p2.run(1.0, sp, ket.d, out->d, ctx.gemm_part.as<double>(), ctx.stream);

@@ -103,9 +103,15 @@ struct GemmPlan {
   double flops = 0.0;
   int64_t c_elems = 0;  // elements of C touched (for traffic accounting)
   bool full = true;     // every enumerated task has work (no empty contraction)
+  // The tilings are made for the path that runs the plan: tiles/reduce of the FP64 pipe,
+  // tiles_tc/reduce_tc of the split tensor-core path.
+  bool f64_ready = false, tc_ready = false;
+  void prepare_f64(cudaStream_t st);
+  void prepare_tc(cudaStream_t st);
   void upload(cudaStream_t st);
   // partial: nslots * 64 * 64 doubles of scratch (may be null when nslots == 0)
-  void run(double alpha, const double* A, const double* B, double* C, double* partial, cudaStream_t st) const;
+  void run(double alpha, const double* A, const double* B, double* C, double* partial, cudaStream_t st);
+  // (after prepare_f64 / prepare_tc)
   size_t partial_bytes() const { return size_t(nslots) * kGemmTile * kGemmTile * sizeof(double); }
   size_t partial_bytes_tc() const { return size_t(nslots_tc) * kTcTileM * kTcTileN * sizeof(double); }
 };

@@ -65,8 +65,6 @@ Shape Shape::conjugate() const {
 void Tensor::set_blocks(const std::vector<int64_t>& sorted_tags) {
   tags = sorted_tags;
   offsets.resize(tags.size());
-  slot.clear();
-  slot.reserve(tags.size() * 2 + 1);
   int64_t off = 0;
   for (size_t b = 0; b < tags.size(); ++b) {
     if (b && tags[b] <= tags[b - 1]) throw Error(kInvalidArgument, "tensor: block tags must be strictly ascending");
@@ -75,7 +73,6 @@ void Tensor::set_blocks(const std::vector<int64_t>& sorted_tags) {
     sh.index(tags[b], idx);
     if (!sh.allowed(idx)) throw Error(kQShapeMismatch, "tensor: block not allowed by its quantum numbers");
     offsets[b] = off;
-    slot[tags[b]] = static_cast<int32_t>(b);
     off += sh.block_size(idx);
   }
   nnz = off;
@@ -182,13 +179,28 @@ std::vector<GemmTaskRef> enumerate_gemm(Trans ta, Trans tb, const Tensor& a, con
   };
   auto arows = rows_of(av);
   auto brows = rows_of(bv);
+  // A result block is allowed where the quantum numbers of its row and column sectors add up
+  // to c.q: the columns by quantum number (ascending), looked up per row
+  auto q_of = [&](int64_t rest, int lo, int hi) {
+    Qn q;
+    for (int k = hi - 1; k >= lo; --k) {
+      const int64_t n = static_cast<int64_t>(c.qshape[k].size());
+      q = q + c.qshape[k][rest % n];
+      rest /= n;
+    }
+    return q;
+  };
+  std::map<Qn, std::vector<size_t>> cols_of;
+  for (size_t y = 0; y < brows.size(); ++y) cols_of[q_of(brows[y].first, L - K, c.rank)].push_back(y);
   std::vector<GemmTaskRef> tasks;
   for (auto& ar : arows) {
     const int64_t i = ar.first;
-    for (auto& br : brows) {
+    const auto cols = cols_of.find(c.q + -q_of(i, 0, L - K));
+    if (cols == cols_of.end()) continue;
+    for (size_t y : cols->second) {
+      const auto& br = brows[y];
       const int64_t j = br.first;
       const int64_t ij = i * colsB + j;
-      if (!c.allowed_tag(ij)) continue;
       GemmTaskRef task;
       task.c_tag = ij;
       // pairs in (aik ascending, bjk ascending) order with equal contracted tag

@@ -8,11 +8,11 @@
 // element offsets and dims so every plan below is pure host integer work.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <map>
 #include <stdexcept>
 #include <string>
-#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -94,7 +94,6 @@ struct Tensor {
   Shape sh;
   std::vector<int64_t> tags;     // ascending
   std::vector<int64_t> offsets;  // element offset of each block
-  std::unordered_map<int64_t, int32_t> slot;
   int64_t nnz = 0;
   double* d = nullptr;  // device data (nnz doubles), owned when own == true
   bool own = false;
@@ -108,9 +107,9 @@ struct Tensor {
 
   void set_blocks(const std::vector<int64_t>& sorted_tags);
   void allocate_allowed();  // every allowed block of non-zero size (STArray.h:219-237)
-  int32_t find(int64_t t) const {
-    auto it = slot.find(t);
-    return it == slot.end() ? -1 : it->second;
+  int32_t find(int64_t t) const {  // block of a tag, -1: not stored
+    auto it = std::lower_bound(tags.begin(), tags.end(), t);
+    return it == tags.end() || *it != t ? -1 : static_cast<int32_t>(it - tags.begin());
   }
   void block_dims(int32_t b, int* dims) const {
     int idx[kMaxRank];
