@@ -1311,7 +1311,7 @@ static void sigma_run_pk(Context& ctx, SigmaPlan& p, const DTensor& L, const DTe
     ctx.timers[kPhSigma] -= tm.dt;  // counted as planning, not as H_eff * psi
   }
   launch_pack(p.pk_psi.packs.get(), static_cast<int>(p.pk_psi.h_packs.size()), psi, p.pk_psi.buf.as<uint8_t>(),
-              ctx.stream);
+              ctx.stream, p.flops < kChainMaxFlops);
   if (p.group_budget < 0) {
     if (ctx.sigma_w_budget < 0) {
       tune_sigma_groups(ctx, p, L, R);
@@ -1347,24 +1347,25 @@ static void sigma_run_pk(Context& ctx, SigmaPlan& p, const DTensor& L, const DTe
 // Both stages over all of w at once (the packed L*psi intermediate in HBM).
 static void sigma_run_pk_whole(Context& ctx, SigmaPlan& p, double* sigma) {
   int* err = device_err_flag(ctx);
+  const bool chained = p.flops < kChainMaxFlops;
   if (p.stack1)
     launch_gemm_pk(p.pk_L.buf.as<uint8_t>(), p.pk_psi.buf.as<uint8_t>(), 1.0, nullptr, p.pk_scr1.buf.as<uint8_t>(),
                    p.st1.get(), static_cast<int>(p.h_st1.size()), p.pk_tasks1.get(), p.stpk1.get(), nullptr,
                    p.scr1_single ? kOutPackedSingle : kOutPackedSplit, p.stage1_single(), err, ctx.stream,
-                   ctx.device_timeout_ns, p.row_map.get());
+                   ctx.device_timeout_ns, p.row_map.get(), chained);
   else
     launch_gemm_pk(p.pk_L.buf.as<uint8_t>(), p.pk_psi.buf.as<uint8_t>(), 1.0, nullptr, p.pk_scr1.buf.as<uint8_t>(),
                    p.s1.tiles_tc.get(), static_cast<int>(p.s1.h_tiles_tc.size()), p.pk_tasks1.get(), p.pk1.get(),
                    nullptr, p.scr1_single ? kOutPackedSingle : kOutPackedSplit, p.stage1_single(), err, ctx.stream,
-                   ctx.device_timeout_ns);
+                   ctx.device_timeout_ns, nullptr, chained);
   ctx.gemm_part.ensure(std::max<size_t>(p.s2.partial_bytes_tc(), 16), ctx.stream);
   double* part = ctx.gemm_part.as<double>();
   launch_gemm_pk(p.pk_scr1.buf.as<uint8_t>(), p.pk_R.buf.as<uint8_t>(), 1.0, sigma, nullptr,
                  p.s2.tiles_tc.get(), static_cast<int>(p.s2.h_tiles_tc.size()), p.s2.dtasks.get(), p.pk2.get(), part,
-                 kOutFP64, p.stage2_single(), err, ctx.stream, ctx.device_timeout_ns);
+                 kOutFP64, p.stage2_single(), err, ctx.stream, ctx.device_timeout_ns, nullptr, chained);
   if (p.s2.nslots_tc > 0)
     launch_gemm_pk_reduce(p.s2.reduce_tc.get(), static_cast<int>(p.s2.h_reduce_tc.size()), p.s2.dtasks.get(), 1.0,
-                          part, sigma, ctx.stream);
+                          part, sigma, ctx.stream, chained);
   ctx.kernel_launches += 3 + (p.s2.nslots_tc > 0);
 }
 
@@ -1373,6 +1374,7 @@ static void sigma_run_pk_whole(Context& ctx, SigmaPlan& p, double* sigma) {
 // operators' digits are kept while their data stays.  False: no memory for it.
 static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTensor& R, const double* psi,
                          double* sigma) {
+  std::vector<OzSource> pack;
   {
     PhaseTimer tm(ctx, kPhSigmaPlan);
     if (!p.o1.built) build_oz_gemm(ctx, p.o1, p.s1, L, p.psi_layout, true);
@@ -1383,7 +1385,7 @@ static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTe
       if (o.src_layout == x.second->layout_id && o.src_version == x.second->data_version &&
           (!x.second->exposed || o.src_call == ctx.call))
         continue;
-      oz_pack(ctx, o, x.second->d);
+      pack.push_back(OzSource{&o, x.second->d});
       o.src_layout = x.second->layout_id;
       o.src_version = x.second->data_version;
       o.src_call = ctx.call;
@@ -1393,9 +1395,10 @@ static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTe
   }
   ctx.scr1.ensure(std::max<int64_t>(p.o1.tiled_elems, 1) * sizeof(double), ctx.stream);
   double* scr = ctx.scr1.as<double>();
-  oz_pack(ctx, p.o1.b, psi);
+  pack.push_back(OzSource{&p.o1.b, psi});
+  oz_pack(ctx, pack);
   run_oz_gemm(ctx, p.o1, p.s1, 1.0, L.d, psi, scr, true);
-  oz_pack(ctx, p.o2.a, scr);
+  oz_pack(ctx, {{&p.o2.a, scr}});
   run_oz_gemm(ctx, p.o2, p.s2, 1.0, scr, R.d, sigma, false);
   return true;
 }
@@ -1722,12 +1725,12 @@ static bool renorm_run_oz(Context& ctx, RenormPlan& rp, const DTensor& bra, cons
   if (!rp.o1.built) build_oz_gemm(ctx, rp.o1, rp.p1, conj_view(bra), opr0);
   if (!rp.o2.built) build_oz_gemm(ctx, rp.o2, rp.p2, rp.scr, ket);
   if (!oz_reserve(ctx, {&rp.o1, &rp.o2})) return false;
-  oz_pack(ctx, rp.o1.swap ? rp.o1.b : rp.o1.a, bra.d);
-  oz_pack(ctx, rp.o1.swap ? rp.o1.a : rp.o1.b, opr0.d);
+  oz_pack(ctx, {{&rp.o1.a, rp.o1.swap ? opr0.d : bra.d},
+                {&rp.o1.b, rp.o1.swap ? bra.d : opr0.d},
+                {rp.o2.swap ? &rp.o2.a : &rp.o2.b, ket.d}});
   if (!rp.p1.full) cuda_check(cudaMemsetAsync(scr, 0, rp.scr.nnz * sizeof(double), ctx.stream), "renorm scr zero");
   run_oz_gemm(ctx, rp.o1, rp.p1, 1.0, bra.d, opr0.d, scr, true);
-  oz_pack(ctx, rp.o2.swap ? rp.o2.b : rp.o2.a, scr);
-  oz_pack(ctx, rp.o2.swap ? rp.o2.a : rp.o2.b, ket.d);
+  oz_pack(ctx, {{rp.o2.swap ? &rp.o2.b : &rp.o2.a, scr}});
   run_oz_gemm(ctx, rp.o2, rp.p2, 1.0, scr, ket.d, out, false);
   rp.o1.release();
   rp.o2.release();

@@ -122,6 +122,11 @@ enum Precision : int { kFP64 = 0, kSplitTF32 = 1, kSplitTF32All = 2 };
 
 // target number of CTAs a grouped GEMM is split into (a few waves on 152 SMs)
 constexpr int kTargetCtas = 152 * 8;
+// split H_eff*psi: largest plan whose launches are chained (launch.hpp).  Chained against
+// plain: 74 : 82 us at 0.1 GFLOP (Hubbard M=256), 52 : 58 at 1.5 MFLOP; but 283 : 273 us at 0.4
+// GFLOP (QC n=12 M=120) and 1523 : 1507 at 88 (C2 size).  The sliced FP64 path gains at every
+// size (521 : 561 us at QC n=14 M=120, 7.88 : 7.99 ms at the C2 size).
+constexpr double kChainMaxFlops = 2.0e8;
 // packed L*psi intermediates above this size make the tuner try w-blocked schedules
 constexpr int64_t kGroupIntermediateBytes = int64_t(8) << 30;
 
@@ -226,8 +231,12 @@ struct OzGemm {
 // plan whose tiled result is this one's A (blocks of `a` matched by from's task result tags).
 void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a, const Tensor& b, bool tiled_out = false,
                    const OzGemm* from = nullptr, const GemmPlan* from_plan = nullptr);
-// Packs an operand of a built plan from FP64 data.
-void oz_pack(Context& ctx, OzOperand& o, const double* src);
+// Packs operands of built plans from FP64 data, up to kOzPackJobs in one launch.
+struct OzSource {
+  OzOperand* o;
+  const double* src;
+};
+void oz_pack(Context& ctx, const std::vector<OzSource>& what);
 // C = (assign) or += alpha op(A) op(B) from the packed operands.
 void run_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, double alpha, const double* A, const double* B, double* C,
                  bool assign);

@@ -159,6 +159,7 @@ struct DPack {
 // Every wait of the kernel gives up after timeout_ns (the whole launch): the kernel then
 // drains its own bulk copies and MMAs, frees its tensor memory, sets *err and returns.
 constexpr uint64_t kPkTimeoutNs = 20000000000ull;  // 20 s
+// chained: launched as part of a dependent chain (launch.hpp; not while a graph is captured).
 // row_map (packed output only, may be null): the A tiles stack several blocks' rows (a
 // stacked panel; the pair's pad field is the panel's first entry in row_map); entry
 // (task << 32 | block row) per panel row, -1 for padding rows, says which output block
@@ -166,10 +167,11 @@ constexpr uint64_t kPkTimeoutNs = 20000000000ull;  // 20 s
 void launch_gemm_pk(const uint8_t* Apk, const uint8_t* Bpk, double alpha, double* C, uint8_t* Cpk,
                     const DTile* tiles, int ntiles, const DGemmTask* tasks, const DPkPair* pairs, double* partial,
                     int out_packed, int single, int* err, cudaStream_t st, uint64_t timeout_ns = kPkTimeoutNs,
-                    const int64_t* row_map = nullptr);
+                    const int64_t* row_map = nullptr, bool chained = false);
 void launch_gemm_pk_reduce(const DReduce* red, int nred, const DGemmTask* tasks, double alpha, const double* partial,
-                           double* C, cudaStream_t st);
-void launch_pack(const DPack* packs, int npacks, const double* src, uint8_t* dst, cudaStream_t st);
+                           double* C, cudaStream_t st, bool chained = false);
+void launch_pack(const DPack* packs, int npacks, const double* src, uint8_t* dst, cudaStream_t st,
+                 bool chained = false);
 int pk_smem_bytes();
 
 // ---- FP64 GEMM on the tensor cores (kernels_oz.cu) ------------------------------
@@ -243,8 +245,22 @@ struct OzGemmArgs {
 };
 void launch_gemm_oz(const OzGemmArgs& a, cudaStream_t st);
 void launch_oz_reduce(const DReduce* red, int nred, const OzGemmArgs& a, cudaStream_t st);
-void launch_oz_pack(const DOzPack* packs, int npacks, const DOzSeg* segs, const double* src, uint8_t* dst, int* exps,
-                    int* flag, int seq, cudaStream_t st);
+// Operands packed by one launch: exps one per packed row, flag set to seq where a value cannot
+// be sliced.
+struct OzPackJob {
+  const DOzPack* packs;
+  const DOzSeg* segs;
+  const double* src;
+  uint8_t* dst;
+  int *exps, *flag;
+  int npacks, seq;
+};
+constexpr int kOzPackJobs = 3;
+struct OzPackJobs {
+  OzPackJob job[kOzPackJobs];
+  int n;
+};
+void launch_oz_pack(const OzPackJobs& jobs, cudaStream_t st);
 
 void launch_gemm_f64(int transa, int transb, double alpha, const double* A, const double* B, double* C,
                      const DTile* tiles, int ntiles, const DGemmTask* tasks, const DGemmPair* pairs,

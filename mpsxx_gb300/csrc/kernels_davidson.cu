@@ -6,12 +6,13 @@
 // Bound by latency at small n and by the FP64 pipe at large n (2.1 FMA per clock and SM,
 // about 3 m + 15 operations per element and iteration): a launch is at most 304 CTAs of 128
 // threads whose sums are added in a fixed order by the last CTA to arrive, so that no second
-// kernel is needed.  Sums the host reads are written to mapped host memory as well.  An
+// kernel is needed, and launches are chained.  Sums the host reads are written to mapped host memory as well.  An
 // iteration took 25 launches with rotations and separate reductions on n / 2048 CTAs: 45 us
 // per dot product at n = 16 k, now 4 us.
 #include <cuda_runtime.h>
 
 #include "kernels.hpp"
+#include "launch.hpp"
 
 namespace mpsxx {
 
@@ -59,6 +60,8 @@ __device__ void grid_sums(const double (&acc)[NVMAX], int nv, const DvReduce& rd
 // out[j] = x . Y_j, j < m
 __global__ void __launch_bounds__(DT) dv_dots_kernel(const double* __restrict__ x, const double* __restrict__ Y, int m,
                                                      int64_t n, DvReduce rd) {
+  chain_wait();
+  chain_next();
   double acc[NVMAX] = {};
   for (int64_t e = blockIdx.x * (int64_t)DT + threadIdx.x; e < n; e += (int64_t)gridDim.x * DT) {
     const double a = x[e];
@@ -74,6 +77,8 @@ __global__ void __launch_bounds__(DT) dv_dots_kernel(const double* __restrict__ 
 __global__ void __launch_bounds__(DT) dv_residual_kernel(const double* __restrict__ T, const double* __restrict__ S,
                                                          const double* __restrict__ diag, int m, int64_t n, DvCoef r,
                                                          double e, double* __restrict__ c, DvReduce rd) {
+  chain_wait();
+  chain_next();
   double acc[NVMAX] = {};
   for (int64_t i = blockIdx.x * (int64_t)DT + threadIdx.x; i < n; i += (int64_t)gridDim.x * DT) {
     double tv[kMaxDot], t = 0.0, s = 0.0;
@@ -104,6 +109,8 @@ __global__ void __launch_bounds__(DT) dv_residual_kernel(const double* __restric
 __global__ void __launch_bounds__(DT) dv_project_kernel(const double* __restrict__ T, int m, int64_t n,
                                                         double* __restrict__ c, const double* __restrict__ in, int second,
                                                         DvReduce rd) {
+  chain_wait();
+  chain_next();
   double acc[NVMAX] = {}, p[kMaxDot];
   const double f = second ? 1.0 : 1.0 / sqrt(in[1]);
 #pragma unroll
@@ -131,6 +138,8 @@ __global__ void __launch_bounds__(DT) dv_project_kernel(const double* __restrict
 // t = x / sqrt(in[0]) (t may be x); z = 0 (z may be null)
 __global__ void __launch_bounds__(DT) dv_scaled_copy_kernel(const double* x, int64_t n, const double* __restrict__ in,
                                                             double* t, double* __restrict__ z) {
+  chain_wait();
+  chain_next();
   const double f = 1.0 / sqrt(in[0]);
   for (int64_t i = blockIdx.x * (int64_t)DT + threadIdx.x; i < n; i += (int64_t)gridDim.x * DT) {
     t[i] = f * x[i];
@@ -140,6 +149,8 @@ __global__ void __launch_bounds__(DT) dv_scaled_copy_kernel(const double* x, int
 
 // out = sum_i r_i T_i (out may be T_0)
 __global__ void __launch_bounds__(DT) dv_combine_kernel(const double* T, int m, int64_t n, DvCoef r, double* out) {
+  chain_wait();
+  chain_next();
   for (int64_t i = blockIdx.x * (int64_t)DT + threadIdx.x; i < n; i += (int64_t)gridDim.x * DT) {
     double t = 0.0;
 #pragma unroll
@@ -159,25 +170,25 @@ int dv_blocks(int64_t n) {
 size_t dv_partial_doubles() { return size_t(kMultidotMaxBlocks) * NVMAX; }
 
 void launch_dv_dots(const double* x, const double* Y, int m, int64_t n, const DvReduce& rd, cudaStream_t st) {
-  dv_dots_kernel<<<dv_blocks(n), DT, 0, st>>>(x, Y, m, n, rd);
+  launch_chained(dv_dots_kernel, dim3(dv_blocks(n)), DT, 0, st, x, Y, m, n, rd);
 }
 
 void launch_dv_residual(const double* T, const double* S, const double* diag, int m, int64_t n, const DvCoef& r,
                         double e, double* c, const DvReduce& rd, cudaStream_t st) {
-  dv_residual_kernel<<<dv_blocks(n), DT, 0, st>>>(T, S, diag, m, n, r, e, c, rd);
+  launch_chained(dv_residual_kernel, dim3(dv_blocks(n)), DT, 0, st, T, S, diag, m, n, r, e, c, rd);
 }
 
 void launch_dv_project(const double* T, int m, int64_t n, double* c, const double* in, int second, const DvReduce& rd,
                        cudaStream_t st) {
-  dv_project_kernel<<<dv_blocks(n), DT, 0, st>>>(T, m, n, c, in, second, rd);
+  launch_chained(dv_project_kernel, dim3(dv_blocks(n)), DT, 0, st, T, m, n, c, in, second, rd);
 }
 
 void launch_dv_scaled_copy(const double* x, int64_t n, const double* in, double* t, double* z, cudaStream_t st) {
-  dv_scaled_copy_kernel<<<dv_blocks(n), DT, 0, st>>>(x, n, in, t, z);
+  launch_chained(dv_scaled_copy_kernel, dim3(dv_blocks(n)), DT, 0, st, x, n, in, t, z);
 }
 
 void launch_dv_combine(const double* T, int m, int64_t n, const DvCoef& r, double* out, cudaStream_t st) {
-  dv_combine_kernel<<<dv_blocks(n), DT, 0, st>>>(T, m, n, r, out);
+  launch_chained(dv_combine_kernel, dim3(dv_blocks(n)), DT, 0, st, T, m, n, r, out);
 }
 
 }  // namespace mpsxx

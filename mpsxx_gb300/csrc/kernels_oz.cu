@@ -41,6 +41,7 @@
 #include <cstdint>
 
 #include "kernels.hpp"
+#include "launch.hpp"
 #include "tc.hpp"
 
 namespace mpsxx {
@@ -173,11 +174,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_oz_kernel(const OzGemmArgs g
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
 
-  if (*g.flag_a == g.seq_a || *g.flag_b == g.seq_b) {
-    for (int ti = g.cta_ptr[blockIdx.x]; ti < g.cta_ptr[blockIdx.x + 1]; ++ti) oz_plain_tile(g.tiles[ti], g);
-    return;
-  }
-
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
@@ -202,10 +198,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_oz_kernel(const OzGemmArgs g
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_slot;
+  chain_wait();
+  const bool plain = *g.flag_a == g.seq_a || *g.flag_b == g.seq_b;
   const uint64_t deadline = deadline_in(g.timeout_ns);
   // Persistent: the CTA walks its list of tiles (balanced on the host); every role walks the
   // same sequence, so stage and accumulator counters continue across tiles.
-  const int ti0 = g.cta_ptr[blockIdx.x], ti1 = g.cta_ptr[blockIdx.x + 1];
+  const int ti0 = g.cta_ptr[blockIdx.x], ti1 = plain ? ti0 : g.cta_ptr[blockIdx.x + 1];
+  if (plain)
+    for (int ti = ti0; ti < g.cta_ptr[blockIdx.x + 1]; ++ti) oz_plain_tile(g.tiles[ti], g);
   if (warp == 0) {
     // ---------------- producer ----------------
     if (lane == 0) {
@@ -422,6 +422,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_oz_kernel(const OzGemmArgs g
       }
     }
   }
+  chain_next();
   __syncthreads();
   if (threadIdx.x == 0 && abort_flag) report_timeout(g.err);
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -432,6 +433,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_oz_kernel(const OzGemmArgs g
 
 // Split-K partials of one tile summed into C in slot order, one thread per valid element.
 __global__ void __launch_bounds__(256) oz_reduce_kernel(const DReduce* __restrict__ red, const OzGemmArgs g) {
+  chain_wait();
+  chain_next();
   const DReduce rd = red[blockIdx.x];
   const DGemmTask tk = g.tasks[rd.task];
   const int rows = g.swap ? tk.n : tk.m, cols = g.swap ? tk.m : tk.n;
@@ -480,14 +483,19 @@ __device__ __forceinline__ unsigned long long biased56(double x, int e1022) {
 // bytes per element; the integer pipe works about 45 instructions on one, which is why the
 // digits are cut by byte permutes and one FP32 addition each.
 constexpr int kHold = 2;
-__global__ void __launch_bounds__(256, 3) oz_pack_kernel(const DOzPack* __restrict__ packs,
-                                                         const DOzSeg* __restrict__ segs, const double* __restrict__ src,
-                                                         uint8_t* __restrict__ dst, int* __restrict__ exps,
-                                                         int* __restrict__ flag, int seq) {
+__global__ void __launch_bounds__(256, 3) oz_pack_kernel(const OzPackJobs jobs) {
   __shared__ long long row_off[kOzPackRows];
   __shared__ int row_ks[kOzPackRows];
   __shared__ int row_max[kOzPackRows];
-  const DOzPack pk = packs[blockIdx.x];
+  chain_wait();
+  chain_next();
+  int first = 0, jb = 0;  // the CTA's operand and its place among that operand's packs
+  while (jb + 1 < jobs.n && (int)blockIdx.x - first >= jobs.job[jb].npacks) first += jobs.job[jb++].npacks;
+  const OzPackJob& job = jobs.job[jb];
+  const DOzSeg* __restrict__ segs = job.segs;
+  const double* __restrict__ src = job.src;
+  uint8_t* __restrict__ dst = job.dst;
+  const DOzPack pk = job.packs[blockIdx.x - first];
   if (threadIdx.x < pk.rows) {
     const int r = threadIdx.x;
     long long off = -1;
@@ -586,8 +594,8 @@ __global__ void __launch_bounds__(256, 3) oz_pack_kernel(const DOzPack* __restri
   __syncthreads();
   if (threadIdx.x < pk.rows) {
     const int e = row_exponent(row_max[threadIdx.x] >> 20);
-    exps[pk.exp0 + threadIdx.x] = e;
-    if (e > kOzMaxExponent) atomicMax(flag, seq);  // (a value that is not finite has the largest exponent)
+    job.exps[pk.exp0 + threadIdx.x] = e;
+    if (e > kOzMaxExponent) atomicMax(job.flag, job.seq);  // (a value that is not finite has the largest exponent)
   }
 #pragma unroll
   for (int h = 0; h < kHold; ++h)
@@ -610,18 +618,19 @@ void launch_gemm_oz(const OzGemmArgs& a, cudaStream_t st) {
     cudaFuncSetAttribute(gemm_oz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     ready = true;
   }
-  gemm_oz_kernel<<<a.nctas, NTHREADS, SMEM_BYTES, st>>>(a);
+  launch_chained(gemm_oz_kernel, dim3(a.nctas), NTHREADS, SMEM_BYTES, st, a);
 }
 
 void launch_oz_reduce(const DReduce* red, int nred, const OzGemmArgs& a, cudaStream_t st) {
   if (nred <= 0) return;
-  oz_reduce_kernel<<<dim3(nred, (OM * ON) / 256), 256, 0, st>>>(red, a);
+  launch_chained(oz_reduce_kernel, dim3(nred, (OM * ON) / 256), 256, 0, st, red, a);
 }
 
-void launch_oz_pack(const DOzPack* packs, int npacks, const DOzSeg* segs, const double* src, uint8_t* dst, int* exps,
-                    int* flag, int seq, cudaStream_t st) {
-  if (npacks <= 0) return;
-  oz_pack_kernel<<<npacks, 256, 0, st>>>(packs, segs, src, dst, exps, flag, seq);
+void launch_oz_pack(const OzPackJobs& jobs, cudaStream_t st) {
+  int n = 0;
+  for (int i = 0; i < jobs.n; ++i) n += jobs.job[i].npacks;
+  if (n <= 0) return;
+  launch_chained(oz_pack_kernel, dim3(n), 256, 0, st, jobs);
 }
 
 }  // namespace mpsxx

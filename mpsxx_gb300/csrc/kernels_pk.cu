@@ -37,6 +37,7 @@
 #include <cstdint>
 
 #include "kernels.hpp"
+#include "launch.hpp"
 #include "tc.hpp"
 
 namespace mpsxx {
@@ -164,6 +165,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_slot;
+  chain_wait();
   const uint64_t deadline = deadline_in(timeout_ns);
   const bool a_single = single & kSingleA, b_single = single & kSingleB;
   const int conv = single & (kSingleA | kSingleB);
@@ -481,6 +483,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
     }
   }
+  chain_next();
   __syncthreads();
   if (threadIdx.x == 0 && abort_flag) report_timeout(err);
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -492,6 +495,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // Pack FP64 blocks into split-TF32 tiles: one CTA per output tile.
 __global__ void __launch_bounds__(256) pack_kernel(const DPack* __restrict__ packs, const double* __restrict__ src,
                                                    uint8_t* __restrict__ dst) {
+  chain_wait();
+  chain_next();
   const DPack pk = packs[blockIdx.x];
   const int rows_t = pk.tile_rows;
   const uint32_t half = (uint32_t)rows_t * BK * 4;  // bytes of one half (hi or lo) of the tile
@@ -529,6 +534,8 @@ __global__ void __launch_bounds__(256) gemm_pk_reduce_kernel(const DReduce* __re
                                                              const DGemmTask* __restrict__ tasks, double alpha,
                                                              const double* __restrict__ partial,
                                                              double* __restrict__ C) {
+  chain_wait();
+  chain_next();
   const DReduce rd = red[blockIdx.x];
   const DGemmTask task = tasks[rd.task];
   const int m0 = rd.tm * BM, n0 = rd.tn * BN;
@@ -557,7 +564,7 @@ int pk_smem_bytes() { return SMEM_BYTES; }
 void launch_gemm_pk(const uint8_t* Apk, const uint8_t* Bpk, double alpha, double* C, uint8_t* Cpk,
                     const DTile* tiles, int ntiles, const DGemmTask* tasks, const DPkPair* pairs, double* partial,
                     int out_packed, int single, int* err, cudaStream_t st, uint64_t timeout_ns,
-                    const int64_t* row_map) {
+                    const int64_t* row_map, bool chained) {
   if (ntiles <= 0) return;
   static int nsm = 0;
   if (nsm == 0) {
@@ -569,19 +576,30 @@ void launch_gemm_pk(const uint8_t* Apk, const uint8_t* Bpk, double alpha, double
   }
   // one persistent CTA per SM; the bound covers the whole launch, not one tile
   const int grid = ntiles < nsm ? ntiles : nsm;
-  gemm_pk_kernel<<<grid, NTHREADS, SMEM_BYTES, st>>>(Apk, Bpk, alpha, C, Cpk, tiles, ntiles, tasks, pairs, partial,
-                                                     out_packed, single, err, timeout_ns, row_map);
+  if (chained)
+    launch_chained(gemm_pk_kernel, dim3(grid), NTHREADS, SMEM_BYTES, st, Apk, Bpk, alpha, C, Cpk, tiles, ntiles, tasks,
+                   pairs, partial, out_packed, single, err, timeout_ns, row_map);
+  else
+    gemm_pk_kernel<<<grid, NTHREADS, SMEM_BYTES, st>>>(Apk, Bpk, alpha, C, Cpk, tiles, ntiles, tasks, pairs, partial,
+                                                       out_packed, single, err, timeout_ns, row_map);
 }
 
-void launch_pack(const DPack* packs, int npacks, const double* src, uint8_t* dst, cudaStream_t st) {
+void launch_pack(const DPack* packs, int npacks, const double* src, uint8_t* dst, cudaStream_t st, bool chained) {
   if (npacks <= 0) return;
-  pack_kernel<<<npacks, 256, 0, st>>>(packs, src, dst);
+  if (chained)
+    launch_chained(pack_kernel, dim3(npacks), 256, 0, st, packs, src, dst);
+  else
+    pack_kernel<<<npacks, 256, 0, st>>>(packs, src, dst);
 }
 
 void launch_gemm_pk_reduce(const DReduce* red, int nred, const DGemmTask* tasks, double alpha, const double* partial,
-                           double* C, cudaStream_t st) {
+                           double* C, cudaStream_t st, bool chained) {
   if (nred <= 0) return;
-  gemm_pk_reduce_kernel<<<dim3(nred, (BM * BN) / 256), 256, 0, st>>>(red, tasks, alpha, partial, C);
+  const dim3 grid(nred, (BM * BN) / 256);
+  if (chained)
+    launch_chained(gemm_pk_reduce_kernel, grid, 256, 0, st, red, tasks, alpha, partial, C);
+  else
+    gemm_pk_reduce_kernel<<<grid, 256, 0, st>>>(red, tasks, alpha, partial, C);
 }
 
 }  // namespace mpsxx

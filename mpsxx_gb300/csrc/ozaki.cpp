@@ -271,10 +271,16 @@ bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs) {
   return true;
 }
 
-void oz_pack(Context& ctx, OzOperand& o, const double* src) {
-  ++o.seq;
-  launch_oz_pack(o.packs.get(), static_cast<int>(o.h_packs.size()), o.segs.get(), src, o.buf.as<uint8_t>(),
-                 o.exps.as<int>(), o.exps.as<int>() + o.rows, o.seq, ctx.stream);
+void oz_pack(Context& ctx, const std::vector<OzSource>& what) {
+  if (what.size() > kOzPackJobs) throw Error(kInternal, "sliced gemm: too many operands in one packing");
+  OzPackJobs jobs{};
+  for (const OzSource& w : what) {
+    OzOperand& o = *w.o;
+    ++o.seq;
+    jobs.job[jobs.n++] = OzPackJob{o.packs.get(), o.segs.get(), w.src, o.buf.as<uint8_t>(), o.exps.as<int>(),
+                                   o.exps.as<int>() + o.rows, static_cast<int>(o.h_packs.size()), o.seq};
+  }
+  launch_oz_pack(jobs, ctx.stream);
   ctx.kernel_launches += 1;
 }
 
