@@ -24,8 +24,8 @@
 // next group of K steps issues.
 //
 // H_eff*psi at the C2 size (QC n=20 M=512, 88 GFLOP): 91.5 ms on the FP64 pipe (0.96 TFLOP/s,
-// 89 % of cuBLAS DGEMM), 7.9 ms sliced with both operators packed anew (11 TFLOP/s; GEMMs 5.6
-// ms, packing 2.4), 158 us against 1.25 ms at Hubbard M=512.
+// 89 % of cuBLAS DGEMM), 7.7 ms sliced with both operators packed anew (11 TFLOP/s; GEMMs 5.5
+// ms, packing 2.2), 137 us against 1.25 ms at Hubbard M=512.
 //
 // GEMM CTA (640 threads, warp-specialised, persistent over the tile list): warp 0 lane 0
 // copies operand slices (one bulk copy each of A and B per K step) into a six-stage
@@ -481,9 +481,12 @@ __device__ __forceinline__ unsigned long long biased56(double x, int e1022) {
 // reads whole sectors and its stores fill 128-byte lines; up to kHold items stay in registers
 // between the two steps, what a long row has beyond is read again (from L2).  HBM moves 8 + 14
 // bytes per element; the integer pipe works about 45 instructions on one, which is why the
-// digits are cut by byte permutes and one FP32 addition each.
+// digits are cut by byte permutes and one FP32 addition each.  Both meet in the middle (HBM 65 %,
+// issue 50 %), so that warps in flight decide: four CTAs an SM (64 registers) against three, 2254 ->
+// 2199 us for a renormalisation at QC n=20 M=512 and 7.88 -> 7.68 ms for its H_eff*psi; five with one
+// item held lose it again to the second reads (2394 us, 7.97 ms).
 constexpr int kHold = 2;
-__global__ void __launch_bounds__(256, 3) oz_pack_kernel(const OzPackJobs jobs) {
+__global__ void __launch_bounds__(256, 4) oz_pack_kernel(const OzPackJobs jobs) {
   __shared__ long long row_off[kOzPackRows];
   __shared__ int row_ks[kOzPackRows];
   __shared__ int row_max[kOzPackRows];
