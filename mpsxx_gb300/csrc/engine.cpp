@@ -1731,7 +1731,10 @@ static bool renorm_run_oz(Context& ctx, RenormPlan& rp, const DTensor& bra, cons
   if (!rp.p1.full) cuda_check(cudaMemsetAsync(scr, 0, rp.scr.nnz * sizeof(double), ctx.stream), "renorm scr zero");
   run_oz_gemm(ctx, rp.o1, rp.p1, 1.0, bra.d, opr0.d, scr, true);
   oz_pack(ctx, {{rp.o2.swap ? &rp.o2.b : &rp.o2.a, scr}});
-  run_oz_gemm(ctx, rp.o2, rp.p2, 1.0, scr, ket.d, out, false);
+  // (the result is new: its blocks are written, not added to, and zeroed only where some have
+  // no contribution)
+  if (rp.p2.c_elems != rp.out.nnz) cuda_check(cudaMemsetAsync(out, 0, rp.out.nnz * sizeof(double), ctx.stream), "renorm zero");
+  run_oz_gemm(ctx, rp.o2, rp.p2, 1.0, scr, ket.d, out, true);
   rp.o1.release();
   rp.o2.release();
   return true;
@@ -1752,22 +1755,23 @@ std::unique_ptr<DTensor> renormalize(Context& ctx, bool forward, const DTensor& 
   tplan.stop();
   PhaseTimer trun(ctx, kPhRenormRun);
   out->ctx = &ctx;
-  out->alloc_device(ctx.stream, true);
+  out->alloc_device(ctx.stream, false);
   const int64_t scr_nnz = rp.scr.nnz;
   ctx.scr2.ensure(std::max<int64_t>(scr_nnz, 1) * sizeof(double), ctx.stream);
   double* sp = ctx.scr2.as<double>();
-  auto zero_scr = [&] {
+  auto zero = [&] {
     if (scr_nnz) cuda_check(cudaMemsetAsync(sp, 0, scr_nnz * sizeof(double), ctx.stream), "renorm scr zero");
+    if (out->nnz) cuda_check(cudaMemsetAsync(out->d, 0, out->nnz * sizeof(double), ctx.stream), "renorm zero");
   };
   if (split) {
-    zero_scr();
+    zero();
     run_split_gemm(ctx, rp.g1, rp.p1, 1.0, bra.d, opr0.d, sp);
     run_split_gemm(ctx, rp.g2, rp.p2, 1.0, sp, ket.d, out->d);
     for (Packed* P : {&rp.g1.pa, &rp.g1.pb, &rp.g2.pa, &rp.g2.pb}) P->buf.release();
     check_device_error(ctx);
   } else if (oz_wanted(ctx, rp.p1.flops + rp.p2.flops) && renorm_run_oz(ctx, rp, bra, opr0, ket, sp, out->d)) {
   } else {
-    zero_scr();
+    zero();
     rp.p1.prepare_f64(ctx.stream);
     rp.p2.prepare_f64(ctx.stream);
     ctx.gemm_part.ensure(std::max(rp.p1.partial_bytes(), rp.p2.partial_bytes()), ctx.stream);
