@@ -193,6 +193,8 @@ __global__ void copy_kernel(const DCopy* __restrict__ tasks, const double* __res
 // QC n=20 M=512 (424 M contributions, 1.2 GB): 1.16 ms, after 1.11 ms and 0.2 ms of zeroing
 // with a CTA per sub-block, a division per element and read-modify-write.  Loading a source
 // ahead, or 2 or 8 elements per lane, made no difference.
+// Where there are too few sub-blocks to fill the chip, gridDim.y warps share one, every
+// gridDim.y-th run of 128 elements each (see launch_scatter).
 constexpr int kScatterUnroll = 4;
 __global__ void __launch_bounds__(256, 6) scatter_kernel(const DScatterDst* __restrict__ dsts, int ndst,
                                                       const DScatterSrc* __restrict__ srcs,
@@ -203,7 +205,12 @@ __global__ void __launch_bounds__(256, 6) scatter_kernel(const DScatterDst* __re
   const int n = t.rows * t.cols;
   const int dr = 32 / t.cols, dc = 32 - dr * t.cols;  // 32 elements on, in rows and columns
   int r = lane / t.cols, c = lane - r * t.cols;
-  for (int e = lane; e < n; e += 32 * kScatterUnroll) {
+  const int parts = gridDim.y;
+  for (int e = lane + 32 * kScatterUnroll * blockIdx.y; e < n; e += 32 * kScatterUnroll * parts) {
+    if (parts > 1) {
+      r = e / t.cols;
+      c = e - r * t.cols;
+    }
     double acc[kScatterUnroll] = {};
     for (int s = t.s0; s < t.s1; ++s) {
       const DScatterSrc q = srcs[s];
@@ -231,32 +238,54 @@ __global__ void __launch_bounds__(256, 6) scatter_kernel(const DScatterDst* __re
   }
 }
 
-// One CTA per destination sub-block; for each of its sources a block-wide dot
-// product with a fixed reduction tree (warp shuffles, then the warp totals in order).
-__global__ void adjoint_scatter_kernel(const DScatterDst* __restrict__ dsts, const DScatterSrc* __restrict__ srcs,
-                                       const double* __restrict__ Y, const double* __restrict__ src,
-                                       double* __restrict__ g) {
-  __shared__ double warp_part[8];
+// One CTA per destination sub-block: for each of its sources the dot product with the
+// sub-block, in a fixed order (lanes, then the warps, then a shuffle tree).  Latency bounds it
+// (a few sources of some thousand elements): the eight warps are divided evenly over up to
+// eight sources, and each lane has four pairs of loads in flight.
+__global__ void __launch_bounds__(256) adjoint_scatter_kernel(const DScatterDst* __restrict__ dsts,
+                                                              const DScatterSrc* __restrict__ srcs,
+                                                              const double* __restrict__ Y,
+                                                              const double* __restrict__ src, double* __restrict__ g) {
+  __shared__ double part_sum[256];
   const DScatterDst t = dsts[blockIdx.x];
   if (t.dst_off < 0) return;
-  const int64_t n = (int64_t)t.rows * t.cols;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (int s = t.s0; s < t.s1; ++s) {
-    const DScatterSrc q = srcs[s];
-    double acc = 0.0;
-    for (int64_t e = threadIdx.x; e < n; e += blockDim.x) {
-      const int r = static_cast<int>(e / t.cols), c = static_cast<int>(e % t.cols);
-      acc = fma(Y[t.dst_off + (int64_t)r * t.dld + c], src[q.src_off + (int64_t)r * q.sld + c], acc);
+  const int n = t.rows * t.cols, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int share = 8;  // warps per source
+  while (share > 1 && 8 / share < t.s1 - t.s0) share >>= 1;
+  const int step = 32 * share, dr = step / t.cols, dc = step - dr * t.cols, part = warp % share;
+  for (int s0 = t.s0; s0 < t.s1; s0 += 8 / share) {
+    const int s = s0 + warp / share;
+    double acc[2] = {};
+    if (s < t.s1) {
+      const DScatterSrc q = srcs[s];
+      int e = part * 32 + lane;
+      int r = e / t.cols, c = e - r * t.cols;
+      for (; e < n; e += 4 * step) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (e + u * step < n)
+            acc[u & 1] = fma(Y[t.dst_off + (int64_t)r * t.dld + c], src[q.src_off + (int64_t)r * q.sld + c], acc[u & 1]);
+          r += dr;
+          c += dc;
+          if (c >= t.cols) {
+            c -= t.cols;
+            ++r;
+          }
+        }
+      }
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) warp_part[warp] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double tot = 0.0;
-      for (int w = 0; w < nwarps; ++w) tot += warp_part[w];
-      g[s] = tot;
+    double v = acc[0] + acc[1];
+    if (share > 1) {
+      part_sum[threadIdx.x] = v;
+      __syncthreads();
+      if (part == 0)
+        for (int w = 1; w < share; ++w) v += part_sum[threadIdx.x + 32 * w];
+      __syncthreads();
     }
-    __syncthreads();
+    if (part == 0 && s < t.s1) {
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) g[s] = v;
+    }
   }
 }
 
@@ -279,13 +308,15 @@ __global__ void eig_factors_kernel(const double* __restrict__ G, const double* _
   }
 }
 
+// A warp per entry: its records' values, summed by the lanes in turn and a shuffle tree.
 __global__ void segment_sum_kernel(const int* __restrict__ ptr, const int* __restrict__ idx,
                                    const double* __restrict__ g, int ne, double* __restrict__ G) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int e = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (e >= ne) return;
   double acc = 0.0;
-  for (int k = ptr[e]; k < ptr[e + 1]; ++k) acc += g[idx[k]];
-  G[e] = acc;
+  for (int k = ptr[e] + lane; k < ptr[e + 1]; k += 32) acc += g[idx[k]];
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if (lane == 0) G[e] = acc;
 }
 
 // diag[a, b] += sum_p L_p[a, a] R_p[b, b] over a block's (L, R) pairs, summed in order.  A
@@ -467,7 +498,10 @@ void launch_copy(const DCopy* tasks, int ntasks, const double* src, double* dst,
 void launch_scatter(const DScatterDst* dsts, int ndst, const DScatterSrc* srcs, const double* src, double* dst,
                     cudaStream_t st) {
   if (ndst <= 0) return;
-  scatter_kernel<<<(ndst + 7) / 8, 256, 0, st>>>(dsts, ndst, srcs, src, dst);
+  // warps per sub-block: four waves of warps (48 on each of 152 SMs) where there are sub-blocks
+  // for less, since a warp alone on a sub-block of 98 x 98 takes 40 us
+  const int parts = std::min(16, std::max(1, 4 * 48 * 152 / ndst));
+  scatter_kernel<<<dim3((ndst + 7) / 8, parts), 256, 0, st>>>(dsts, ndst, srcs, src, dst);
 }
 
 void launch_adjoint_scatter(const DScatterDst* dsts, int ndst, const DScatterSrc* srcs, const double* Y,
@@ -486,7 +520,7 @@ void launch_eig_factors(const double* G, const double* w, int d, int k, int tran
 
 void launch_segment_sum(const int* ptr, const int* idx, const double* g, int ne, double* G, cudaStream_t st) {
   if (ne <= 0) return;
-  segment_sum_kernel<<<(ne + 255) / 256, 256, 0, st>>>(ptr, idx, g, ne, G);
+  segment_sum_kernel<<<(ne + 7) / 8, 256, 0, st>>>(ptr, idx, g, ne, G);
 }
 
 void launch_diag(const DDiagTile* tiles, int ntiles, const DDiagTask* tasks, const DDiagPair* pairs, const double* L,
