@@ -188,17 +188,18 @@ __global__ void copy_kernel(const DCopy* __restrict__ tasks, const double* __res
 // environment block, contiguous like the sub-block's rows x cols) in fixed order, or zero.
 // The sub-blocks tile the result, which is written once.  One warp per sub-block, its lanes
 // over consecutive elements, so that a source is read in whole lines and few lanes idle: the
-// FP64 pipe (one multiply-add per contribution, 15 clocks of an SM per warp; a leading
-// coefficient of 1 costs none) bounds the kernel: active 67 % of the time at QC n=16 M=300.
-// QC n=20 M=512 (424 M contributions, 1.2 GB): 1.16 ms, after 1.11 ms and 0.2 ms of zeroing
-// with a CTA per sub-block, a division per element and read-modify-write.  Loading a source
-// ahead, or 2 or 8 elements per lane, made no difference.
-// Where there are too few sub-blocks to fill the chip, gridDim.y warps share one, every
-// gridDim.y-th run of 128 elements each (see launch_scatter).
-constexpr int kScatterUnroll = 4;
-__global__ void __launch_bounds__(256, 6) scatter_kernel(const DScatterDst* __restrict__ dsts, int ndst,
-                                                      const DScatterSrc* __restrict__ srcs,
-                                                      const double* __restrict__ src, double* __restrict__ dst) {
+// FP64 pipe bounds the kernel (one multiply-add per contribution, 15 clocks of an SM per warp;
+// a leading coefficient of 1 costs none, and whether it is one is asked of the integer pipe:
+// with a comparison of doubles per source the calls below took 1357, 1221 and 279 us).
+// Elements per lane and CTAs per SM, QC n=20 M=512 forward (424 M contributions, 1.2 GB) /
+// backward / n=14 M=256, us: 3 x 32 and 4 1009 / 965 / 205, 3 and 5 1066 / 949 / 219, 4 and 6
+// 1150 / 993 / 238, 4 and 4 1018 / 1001 / 213, 2 and 5 1106 / 945 / 219.
+// Where there are too few sub-blocks to fill the chip, gridDim.y warps share one, in turn by
+// the 32 kScatterUnroll elements (see launch_scatter).
+constexpr int kScatterUnroll = 3;
+__global__ void __launch_bounds__(256, 4) scatter_kernel(const DScatterDst* __restrict__ dsts, int ndst,
+                                                         const DScatterSrc* __restrict__ srcs,
+                                                         const double* __restrict__ src, double* __restrict__ dst) {
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= ndst) return;
   const DScatterDst t = dsts[i];
@@ -212,18 +213,25 @@ __global__ void __launch_bounds__(256, 6) scatter_kernel(const DScatterDst* __re
       c = e - r * t.cols;
     }
     double acc[kScatterUnroll] = {};
-    for (int s = t.s0; s < t.s1; ++s) {
+    if (t.s0 < t.s1) {
+      const DScatterSrc q = srcs[t.s0];
+      const double* p = src + q.src_off + e;
+#pragma unroll
+      for (int u = 0; u < kScatterUnroll; ++u)
+        if (e + 32 * u < n) acc[u] = p[32 * u];
+      // (compared as integers: a comparison of doubles is work for the FP64 pipe as well)
+      if (__double2hiint(q.coef) != 0x3ff00000 || __double2loint(q.coef) != 0) {
+#pragma unroll
+        for (int u = 0; u < kScatterUnroll; ++u)
+          if (e + 32 * u < n) acc[u] *= q.coef;
+      }
+    }
+    for (int s = t.s0 + 1; s < t.s1; ++s) {
       const DScatterSrc q = srcs[s];
       const double* p = src + q.src_off + e;
-      if (s == t.s0 && q.coef == 1.0) {
 #pragma unroll
-        for (int u = 0; u < kScatterUnroll; ++u)
-          if (e + 32 * u < n) acc[u] = p[32 * u];
-      } else {
-#pragma unroll
-        for (int u = 0; u < kScatterUnroll; ++u)
-          if (e + 32 * u < n) acc[u] = fma(q.coef, p[32 * u], acc[u]);
-      }
+      for (int u = 0; u < kScatterUnroll; ++u)
+        if (e + 32 * u < n) acc[u] = fma(q.coef, p[32 * u], acc[u]);
     }
 #pragma unroll
     for (int u = 0; u < kScatterUnroll; ++u) {
