@@ -330,11 +330,13 @@ __global__ void segment_sum_kernel(const int* __restrict__ ptr, const int* __res
 // diag[a, b] += sum_p L_p[a, a] R_p[b, b] over a block's (L, R) pairs, summed in order.  A
 // CTA takes up to 256 outputs of a block, w columns (the block's width rounded up to a power
 // of two, at most 32) by 256 / w rows (at most 64), one output per thread, so that lanes idle
-// only at ragged edges; the tied diagonals of 32 pairs at a time are gathered into shared memory while the
-// pairs before them are summed.  Bound by the FP64 pipe (one multiply-add per output and
-// pair, 13 us at QC n=16 M=256) and the gathers' latency: 45 us there, 108 us with 32 x 32
-// tiles of four outputs per thread (few CTAs, half of their lanes on padding).
-constexpr int kDiagPairs = 32;
+// only at ragged edges; the tied diagonals of 16 pairs at a time are gathered into shared
+// memory, each warp's loads in flight together, while the pairs before them are summed.  Bound
+// by the FP64 pipe (one multiply-add per output and pair): at QC n=16 M=256 the call takes 63 us,
+// 44 with one multiply-add per 16 pairs and 32 for a problem of any small size; 66 with 32
+// pairs gathered one after another, 135 with 32 x 32 tiles of four outputs per thread (few
+// CTAs, half of their lanes on padding).
+constexpr int kDiagPairs = 16;
 __global__ void __launch_bounds__(256) diag_kernel(const DDiagTile* __restrict__ tiles,
                                                    const DDiagTask* __restrict__ tasks,
                                                    const DDiagPair* __restrict__ pairs, const double* __restrict__ L,
@@ -346,13 +348,24 @@ __global__ void __launch_bounds__(256) diag_kernel(const DDiagTile* __restrict__
   const int x = threadIdx.x & (w - 1), y = threadIdx.x >> tl.log2w;
   auto gather = [&](int p0, double* s) {
     const int np = min(kDiagPairs, t.p1 - p0);
-    for (int q = threadIdx.x >> 5; q < np; q += 8) {  // a warp per pair
-      const DDiagPair pr = pairs[p0 + q];
-      for (int e = threadIdx.x & 31; e < span; e += 32) {
-        const int a = tl.a0 + e, b = tl.b0 + e - h;
-        s[q * span + e] = e < h ? (a < t.m ? L[pr.l_off + (int64_t)a * (t.m + 1)] : 0.0)
-                                : (b < t.n ? R[pr.r_off + (int64_t)b * (t.n + 1)] : 0.0);
-      }
+    // a warp takes four pairs, their loads in flight together
+    const int q0 = threadIdx.x >> 5;
+    DDiagPair pr[kDiagPairs / 8];
+#pragma unroll
+    for (int i = 0; i < kDiagPairs / 8; ++i)
+      if (q0 + 8 * i < np) pr[i] = pairs[p0 + q0 + 8 * i];
+    for (int e = threadIdx.x & 31; e < span; e += 32) {
+      const int a = tl.a0 + e, b = tl.b0 + e - h;
+      const bool left = e < h, in = left ? a < t.m : b < t.n;
+      const double* base = left ? L : R;
+      const int64_t off = left ? (int64_t)a * (t.m + 1) : (int64_t)b * (t.n + 1);
+      double v[kDiagPairs / 8];
+#pragma unroll
+      for (int i = 0; i < kDiagPairs / 8; ++i)
+        v[i] = in && q0 + 8 * i < np ? base[(left ? pr[i].l_off : pr[i].r_off) + off] : 0.0;
+#pragma unroll
+      for (int i = 0; i < kDiagPairs / 8; ++i)
+        if (q0 + 8 * i < np) s[(q0 + 8 * i) * span + e] = v[i];
     }
   };
   double acc = 0.0;
