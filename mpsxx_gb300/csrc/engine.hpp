@@ -50,6 +50,13 @@ struct DevArray {
   T* get() const { return buf.as<T>(); }
 };
 
+// An array inside a buffer shared by several.
+template <class T>
+struct DevView {
+  T* p = nullptr;
+  T* get() const { return p; }
+};
+
 struct Context;
 
 // Queued host-to-device copy of a small host array through pinned staging memory (the
@@ -177,13 +184,14 @@ struct SplitGemm {
 
 // One operand of a sliced FP64 GEMM: its digit tiles, row exponents and what they hold.
 struct OzOperand {
-  DevBuf buf, exps;  // exps: one exponent per packed row, then the flag
+  DevBuf buf, exps;  // digits; one exponent per packed row
   std::vector<int64_t> base;  // per block slot: byte offset of its tile grid (-1: not packed)
   std::vector<int> exp0, nks;  // per block slot: first exponent, K slices
   std::vector<DOzPack> h_packs;
   std::vector<DOzSeg> h_segs;
-  DevArray<DOzPack> packs;
-  DevArray<DOzSeg> segs;
+  DevView<DOzPack> packs;
+  DevView<DOzSeg> segs;
+  DevView<int> flag;  // number of the last packing that met a value which cannot be sliced
   int64_t bytes = 0;
   int rows = 0;
   int seq = 0;  // packings so far
@@ -206,19 +214,20 @@ struct OzGemm {
   OzOperand a, b;  // row operand (128-row tiles) and column operand (32-row tiles)
   std::vector<DTile> h_tiles;  // by CTA
   std::vector<int> h_cta_ptr;
-  DevArray<DTile> tiles;
-  DevArray<int> cta_ptr;
-  DevArray<DOzPair> pairs;
-  DevArray<int64_t> row_map;
+  DevBuf arrays;  // all device arrays of the plan
+  DevView<DTile> tiles;
+  DevView<int> cta_ptr;
+  DevView<DOzPair> pairs;
+  DevView<int64_t> row_map;
   std::vector<DReduce> h_reduce;
-  DevArray<DReduce> reduce;
+  DevView<DReduce> reduce;
   int nslots = 0;
   // tiled intermediate between two plans: where the first one's tasks go, the size, and
   // the per-pair places (of the panels, or of the second one's row operand blocks)
   bool tiled_out = false, tiled_in = false;
   std::vector<DOzTiled> task_place;
   int64_t tiled_elems = 0;
-  DevArray<DOzTiled> pairs_tiled;
+  DevView<DOzTiled> pairs_tiled;
   size_t partial_bytes() const { return size_t(nslots) * kOzTileM * kOzTileN * sizeof(double); }
   int64_t device_bytes() const { return a.bytes + b.bytes + 4 * (int64_t(a.rows) + b.rows); }
   bool held() const { return a.buf.p && b.buf.p; }

@@ -1,6 +1,7 @@
 // Host side of the FP64 GEMM on the tensor cores (kernels_oz.cu): packed layouts, stacked
 // panels, tiles and launches of a GemmPlan.
 #include <algorithm>
+#include <cstring>
 #include <map>
 #include <set>
 
@@ -79,10 +80,39 @@ void pack_blocks(OzOperand& o, const Tensor& t, const std::vector<View>& view, b
   }
 }
 
-void upload_operand(Context& ctx, OzOperand& o) {
-  o.packs.upload(o.h_packs, ctx.stream);
-  o.segs.upload(o.h_segs, ctx.stream);
-}
+// Host arrays into one device buffer: a small plan's in one copy (a copy's few microseconds
+// are what the first call on a new layout waits for), a large one's each by itself.
+class Upload {
+ public:
+  template <class T>
+  void add(DevView<T>& to, const std::vector<T>& from) {
+    items_.push_back({reinterpret_cast<void**>(&to.p), from.data(), from.size() * sizeof(T), bytes_});
+    bytes_ += (from.size() * sizeof(T) + kAlign) / kAlign * kAlign;
+  }
+  void run(DevBuf& buf, cudaStream_t st) {
+    buf.ensure(bytes_, st);
+    std::vector<char> joined(bytes_ <= kJoin ? bytes_ : 0);
+    for (const Item& i : items_) {
+      *i.to = buf.as<char>() + i.at;
+      if (i.bytes == 0) continue;
+      if (joined.empty())
+        upload_staged(*i.to, i.from, i.bytes, st);
+      else
+        std::memcpy(joined.data() + i.at, i.from, i.bytes);
+    }
+    if (!joined.empty()) upload_staged(buf.p, joined.data(), joined.size(), st);
+  }
+
+ private:
+  static constexpr size_t kAlign = 64, kJoin = 256 * 1024;
+  struct Item {
+    void** to;
+    const void* from;
+    size_t bytes, at;
+  };
+  std::vector<Item> items_;
+  size_t bytes_ = 0;
+};
 
 }  // namespace
 
@@ -231,14 +261,20 @@ void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a,
     og.h_cta_ptr.push_back(static_cast<int>(sorted.size()));
   }
   og.h_tiles.swap(sorted);
-  og.tiles.upload(og.h_tiles, ctx.stream);
-  og.cta_ptr.upload(og.h_cta_ptr, ctx.stream);
-  if (!pairs_tiled.empty()) og.pairs_tiled.upload(pairs_tiled, ctx.stream);
-  og.pairs.upload(pairs, ctx.stream);
-  if (og.stacked) og.row_map.upload(row_map, ctx.stream);
-  og.reduce.upload(og.h_reduce, ctx.stream);
-  upload_operand(ctx, og.a);
-  upload_operand(ctx, og.b);
+  const std::vector<int> none{0};
+  Upload up;
+  up.add(og.tiles, og.h_tiles);
+  up.add(og.cta_ptr, og.h_cta_ptr);
+  up.add(og.pairs_tiled, pairs_tiled);
+  up.add(og.pairs, pairs);
+  up.add(og.row_map, row_map);
+  up.add(og.reduce, og.h_reduce);
+  for (OzOperand* o : {&og.a, &og.b}) {
+    up.add(o->packs, o->h_packs);
+    up.add(o->segs, o->h_segs);
+    up.add(o->flag, none);
+  }
+  up.run(og.arrays, ctx.stream);
   og.built = true;
 }
 
@@ -258,10 +294,8 @@ bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs) {
   try {
     for (OzGemm* g : gs)
       for (OzOperand* o : {&g->a, &g->b}) {
-        const bool fresh = o->exps.p == nullptr;
         o->buf.ensure(std::max<int64_t>(o->bytes, 16), ctx.stream);
-        o->exps.ensure(size_t(o->rows + 1) * sizeof(int), ctx.stream);
-        if (fresh) cuda_check(cudaMemsetAsync(o->exps.as<int>() + o->rows, 0, sizeof(int), ctx.stream), "flag zero");
+        o->exps.ensure(size_t(std::max(o->rows, 1)) * sizeof(int), ctx.stream);
       }
   } catch (const Error& e) {
     if (e.code != kAlloc) throw;
@@ -278,7 +312,7 @@ void oz_pack(Context& ctx, const std::vector<OzSource>& what) {
     OzOperand& o = *w.o;
     ++o.seq;
     jobs.job[jobs.n++] = OzPackJob{o.packs.get(), o.segs.get(), w.src, o.buf.as<uint8_t>(), o.exps.as<int>(),
-                                   o.exps.as<int>() + o.rows, static_cast<int>(o.h_packs.size()), o.seq};
+                                   o.flag.get(), static_cast<int>(o.h_packs.size()), o.seq};
   }
   launch_oz_pack(jobs, ctx.stream);
   ctx.kernel_launches += 1;
@@ -292,8 +326,8 @@ void run_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, double alpha, cons
   a.Bpk = og.b.buf.as<uint8_t>();
   a.Aexp = og.a.exps.as<int>();
   a.Bexp = og.b.exps.as<int>();
-  a.flag_a = a.Aexp + og.a.rows;
-  a.flag_b = a.Bexp + og.b.rows;
+  a.flag_a = og.a.flag.get();
+  a.flag_b = og.b.flag.get();
   a.seq_a = og.a.seq;
   a.seq_b = og.b.seq;
   a.tiles = og.tiles.get();
