@@ -137,11 +137,13 @@ constexpr double kChainMaxFlops = 2.0e8;
 // packed L*psi intermediates above this size make the tuner try w-blocked schedules
 constexpr int64_t kGroupIntermediateBytes = int64_t(8) << 30;
 
-// sliced FP64 GEMM: output tiles that a plan with long pair lists is split into
+// sliced FP64 GEMM: output tiles that a plan with long pair lists is split into, in tiles per
+// SM.  8 against 16: 7.88 : 7.76 ms at QC n=20 M=512, 523 : 509 us at n=14 M=120, 136 : 133 at
+// Hubbard M=512, but 521 : 543 at QC n=18 M=60; 2 to 4 are slower everywhere.
 constexpr int kOzTargetTiles = 152 * 8;
 // fewest FLOPs of an FP64 plan that runs sliced on the tensor cores.  One call, FP64 pipe
 // against tensor cores: H_eff*psi 67 : 73 us at 0.18 MFLOP (Hubbard M=32), 96 : 79 at 1.5
-// (M=64), 232 : 87 at 24, 1236 : 158 at 780 (M=512); renormalisation 98 : 94 at 0.24, 123 :
+// (M=64), 232 : 87 at 24, 1236 : 135 at 780 (M=512); renormalisation 98 : 94 at 0.24, 123 :
 // 98 at 0.9, 635 : 375 at 4 (QC n=14 M=40); below a megaflop the two more launches of the
 // packing decide.
 constexpr double kOzMinFlops = 1.0e6;

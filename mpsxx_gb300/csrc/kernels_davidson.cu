@@ -6,9 +6,9 @@
 // Bound by latency at small n and by the FP64 pipe at large n (2.1 FMA per clock and SM,
 // about 3 m + 15 operations per element and iteration): a launch is at most 304 CTAs of 128
 // threads whose sums are added in a fixed order by the last CTA to arrive, so that no second
-// kernel is needed, and launches are chained.  Sums the host reads are written to mapped host memory as well.  An
-// iteration took 25 launches with rotations and separate reductions on n / 2048 CTAs: 45 us
-// per dot product at n = 16 k, now 4 us.
+// kernel is needed, and launches are chained.  Sums the host reads are written to mapped host
+// memory as well.  An iteration took 25 launches with rotations and separate reductions on
+// n / 2048 CTAs: 45 us per dot product at n = 16 k, now 4 us.
 #include <cuda_runtime.h>
 
 #include "kernels.hpp"

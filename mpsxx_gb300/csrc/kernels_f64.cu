@@ -1,8 +1,9 @@
 // FP64 kernels of the two-site hot path: grouped block GEMM, block copies,
 // merged-operator scatter, H_eff diagonal, and the Davidson level-1 operations.
 //
-// GB300 (sm_103a) has a very small FP64 pipe, so the FP64 path is FMA-bound on
-// CUDA cores: a 64x64 output tile per 256-thread CTA, 4x4 register micro-tiles,
+// GB300 (sm_103a) has a very small FP64 pipe, so these kernels are FMA-bound on the
+// CUDA cores.  The GEMM here is for small products and for plans whose digits find no memory
+// (the others are sliced onto the tensor cores, kernels_oz.cu): a 64x64 output tile per 256-thread CTA, 4x4 register micro-tiles,
 // operands staged through shared memory in 16-deep K slices; warps own bands of the
 // tile shaped per tile to its valid extent, and bands outside a ragged block skip
 // their FMAs.  Every output tile

@@ -408,7 +408,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_oz_kernel(const OzGemmArgs g
       if (!work || row < 0) continue;
       if (t.slot >= 0 || g.tiled_out) {
         // a whole tile row: 64 contiguous bytes a lane
-        double* base = g.tiled_out ? g.C + oz_tile_off(g.pairs_tiled[t.p0], t.tm, t.tn) : g.partial + (int64_t)t.slot * (OM * ON);
+        double* base = g.tiled_out ? g.C + oz_tile_off(g.pairs_tiled[t.p0], t.tm, t.tn)
+                                   : g.partial + (int64_t)t.slot * (OM * ON);
         double2* part = reinterpret_cast<double2*>(base + row * ON + c0);
 #pragma unroll
         for (int j = 0; j < EPI_COLS / 2; ++j) part[j] = make_double2(acc[2 * j], acc[2 * j + 1]);
