@@ -554,8 +554,10 @@ void build_gemm_plan(GemmPlan& plan, Trans ta, Trans tb, const Tensor& a, const 
 }
 
 void GemmPlan::upload(cudaStream_t st) {
-  dtasks.upload(h_tasks, st);
-  pairs.upload(h_pairs, st);
+  Upload up;
+  up.add(dtasks, h_tasks);
+  up.add(pairs, h_pairs);
+  up.run(arrays, st);
 }
 
 void GemmPlan::prepare_f64(cudaStream_t st) {

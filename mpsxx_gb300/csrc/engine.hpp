@@ -5,6 +5,7 @@
 #include <cublas_v2.h>
 #include <cusolverDn.h>
 
+#include <cstring>
 #include <functional>
 #include <map>
 #include <mutex>
@@ -62,6 +63,42 @@ struct Context;
 // Queued host-to-device copy of a small host array through pinned staging memory (the
 // source may be reused as soon as the call returns).
 void upload_staged(void* dst, const void* src, size_t bytes, cudaStream_t st);
+
+// Host arrays into one device buffer: a small plan's in one copy (a copy's few microseconds
+// are what the first call on a new layout waits for), a large one's each by itself.
+class Upload {
+ public:
+  template <class T>
+  void add(DevView<T>& to, const std::vector<T>& from) {
+    items_.push_back({&to.p, from.data(), from.size() * sizeof(T), bytes_});
+    bytes_ += (from.size() * sizeof(T) + kAlign) / kAlign * kAlign;
+  }
+  void run(DevBuf& buf, cudaStream_t st) {
+    buf.ensure(bytes_, st);
+    std::vector<char> joined(bytes_ <= kJoin ? bytes_ : 0);
+    for (const Item& i : items_) {
+      char* at = buf.as<char>() + i.at;
+      std::memcpy(i.to, &at, sizeof(at));
+      if (i.bytes == 0) continue;
+      if (joined.empty())
+        upload_staged(at, i.from, i.bytes, st);
+      else
+        std::memcpy(joined.data() + i.at, i.from, i.bytes);
+    }
+    if (!joined.empty()) upload_staged(buf.p, joined.data(), joined.size(), st);
+  }
+
+ private:
+  static constexpr size_t kAlign = 64, kJoin = 256 * 1024;
+  struct Item {
+    void* to;  // the view's pointer
+    const void* from;
+    size_t bytes, at;
+  };
+  std::vector<Item> items_;
+  size_t bytes_ = 0;
+};
+
 // Drops a stream (drained, about to be destroyed) from the staging bookkeeping.
 void forget_stream_uploads(cudaStream_t st);
 
@@ -96,8 +133,9 @@ struct GemmPlan {
   std::vector<int64_t> task_ctag;                 // result block tag of each h_tasks entry
   std::vector<DReduce> h_reduce;
   DevArray<DTile> tiles;
-  DevArray<DGemmTask> dtasks;
-  DevArray<DGemmPair> pairs;
+  DevBuf arrays;  // tasks and pairs
+  DevView<DGemmTask> dtasks;
+  DevView<DGemmPair> pairs;
   DevArray<DReduce> reduce;
   int nslots = 0;  // split-K partial tiles
   // tensor-core (split TF32) tiling of the same tasks: 128 x 128 tiles (64-row and

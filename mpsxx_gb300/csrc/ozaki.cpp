@@ -1,7 +1,6 @@
 // Host side of the FP64 GEMM on the tensor cores (kernels_oz.cu): packed layouts, stacked
 // panels, tiles and launches of a GemmPlan.
 #include <algorithm>
-#include <cstring>
 #include <map>
 #include <set>
 
@@ -79,40 +78,6 @@ void pack_blocks(OzOperand& o, const Tensor& t, const std::vector<View>& view, b
     });
   }
 }
-
-// Host arrays into one device buffer: a small plan's in one copy (a copy's few microseconds
-// are what the first call on a new layout waits for), a large one's each by itself.
-class Upload {
- public:
-  template <class T>
-  void add(DevView<T>& to, const std::vector<T>& from) {
-    items_.push_back({reinterpret_cast<void**>(&to.p), from.data(), from.size() * sizeof(T), bytes_});
-    bytes_ += (from.size() * sizeof(T) + kAlign) / kAlign * kAlign;
-  }
-  void run(DevBuf& buf, cudaStream_t st) {
-    buf.ensure(bytes_, st);
-    std::vector<char> joined(bytes_ <= kJoin ? bytes_ : 0);
-    for (const Item& i : items_) {
-      *i.to = buf.as<char>() + i.at;
-      if (i.bytes == 0) continue;
-      if (joined.empty())
-        upload_staged(*i.to, i.from, i.bytes, st);
-      else
-        std::memcpy(joined.data() + i.at, i.from, i.bytes);
-    }
-    if (!joined.empty()) upload_staged(buf.p, joined.data(), joined.size(), st);
-  }
-
- private:
-  static constexpr size_t kAlign = 64, kJoin = 256 * 1024;
-  struct Item {
-    void** to;
-    const void* from;
-    size_t bytes, at;
-  };
-  std::vector<Item> items_;
-  size_t bytes_ = 0;
-};
 
 }  // namespace
 
