@@ -709,6 +709,8 @@ SigmaPlan& sigma_plan(Context& ctx, const Tensor& L, const Tensor& R, const Tens
   build_gemm_plan(p->s2, kNoTrans, kTrans, p->scr1, R, psi, K2, std::move(t2));
   p->s1.upload(ctx.stream);
   p->s2.upload(ctx.stream);
+  p->stacks = p->s1.full;
+  for (const DGemmTask& t : p->s1.h_tasks) p->stacks = p->stacks && t.p1 - t.p0 == 1;
   p->flops = p->s1.flops + p->s2.flops;
   p->bytes_min = 8 * (L.nnz + R.nnz + 2 * psi.nnz);
   p->psi_layout = psi;
@@ -1371,11 +1373,12 @@ static void sigma_run_pk_whole(Context& ctx, SigmaPlan& p, double* sigma) {
   ctx.kernel_launches += 3 + (p.s2.nslots_tc > 0);
 }
 
-// FP64 H_eff * psi on the tensor cores: L psi into the FP64 intermediate (every block has
-// one pair: stacked panels), the intermediate packed, then the sum over w and B'.  The
-// operators' digits are kept while their data stays.  False: no memory for it.
+// FP64 H_eff * psi on the tensor cores: L psi into the FP64 intermediate (stacked panels), the
+// intermediate packed, then the sum over w and B'.  The operators' digits are kept while their
+// data stays.  False: not for these layouts, or no memory for it.
 static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTensor& R, const double* psi,
                          double* sigma) {
+  if (!p.stacks) return false;
   std::vector<OzSource> pack;
   {
     PhaseTimer tm(ctx, kPhSigmaPlan);

@@ -304,6 +304,9 @@ struct SigmaPlan {
   Tensor scr1;  // layout of L*psi
   GemmPlan s1, s2;
   OzGemm o1, o2;  // both stages' FP64 execution on the tensor cores
+  // every L psi block is one product: false where row sectors of psi repeat a quantum number
+  // (several) or have no states (none)
+  bool stacks = false;
   double flops = 0.0;
   int64_t bytes_min = 0;  // 8*(nnz L + nnz R + 2 nnz psi)
   // split-TF32 path over packed operands
