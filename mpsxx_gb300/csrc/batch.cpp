@@ -415,8 +415,7 @@ class Batch {
       if (it_[c].sp->scr1_single != single || it_[c].sp->ops_single != p0.ops_single)
         throw Error(kInternal, "batched sigma: operand formats differ");
     // capture: zero the outputs, pack the inputs, both stages, the split-K sums
-    cudaGraph_t graph = nullptr;
-    cuda_check(cudaStreamBeginCapture(ctx_.stream, cudaStreamCaptureModeThreadLocal), "batch capture");
+    StreamCapture capture(ctx_.stream);
     const int nm = static_cast<int>(members.size());
     launch_bzero(g->probs.get(), nm, g->nmax, vec_.as<double>(), kSlotOut, ctx_.stream);
     launch_pack(g->packs.get(), g->npacks, vec_.as<double>(), arPsi_.as<uint8_t>(), ctx_.stream);
@@ -428,7 +427,7 @@ class Batch {
                    ctx_.device_timeout_ns);
     launch_gemm_pk_reduce(g->red.get(), g->nred, g->k2.get(), 1.0, ctx_.gemm_part.as<double>(), vec_.as<double>(),
                           ctx_.stream);
-    cuda_check(cudaStreamEndCapture(ctx_.stream, &graph), "batch capture end");
+    cudaGraph_t graph = capture.end();
     cudaError_t e = cudaGraphInstantiate(&g->graph, graph, 0);
     cudaGraphDestroy(graph);
     cuda_check(e, "batch graph instantiate");

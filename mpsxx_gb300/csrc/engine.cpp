@@ -1164,11 +1164,10 @@ static void sigma_groups_graph(Context& ctx, SigmaPlan& p, double* sigma) {
                                          ctx.gemm_part.p,  p.staged.p,   err};
   if (!p.graph || ptrs != p.graph_ptrs) {
     p.drop_graph();
-    cudaGraph_t g = nullptr;
-    cuda_check(cudaStreamBeginCapture(ctx.stream, cudaStreamCaptureModeThreadLocal), "graph capture begin");
+    StreamCapture capture(ctx.stream);
     cuda_check(cudaMemsetAsync(p.staged.p, 0, size_t(n) * sizeof(double), ctx.stream), "staged zero");
     sigma_groups_run(ctx, p, p.staged.as<double>());
-    cuda_check(cudaStreamEndCapture(ctx.stream, &g), "graph capture end");
+    cudaGraph_t g = capture.end();
     cudaError_t e = cudaGraphInstantiate(&p.graph, g, 0);
     cudaGraphDestroy(g);
     cuda_check(e, "graph instantiate");

@@ -58,6 +58,29 @@ struct DevView {
   T* get() const { return p; }
 };
 
+// Capture of a stream's work; one that is left by an exception is ended and dropped.
+class StreamCapture {
+ public:
+  explicit StreamCapture(cudaStream_t st) : st_(st) {
+    cuda_check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "graph capture begin");
+  }
+  StreamCapture(const StreamCapture&) = delete;
+  ~StreamCapture() {
+    cudaGraph_t g = nullptr;
+    if (open_ && cudaStreamEndCapture(st_, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+  }
+  cudaGraph_t end() {
+    cudaGraph_t g = nullptr;
+    open_ = false;
+    cuda_check(cudaStreamEndCapture(st_, &g), "graph capture end");
+    return g;
+  }
+
+ private:
+  cudaStream_t st_;
+  bool open_ = true;
+};
+
 struct Context;
 
 // Queued host-to-device copy of a small host array through pinned staging memory (the

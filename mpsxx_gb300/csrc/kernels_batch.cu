@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "kernels.hpp"
+#include "launch.hpp"
 
 namespace mpsxx {
 namespace {
@@ -212,46 +213,46 @@ int grid_x(int64_t nmax) { return static_cast<int>(std::max<int64_t>(1, std::min
 
 void launch_bcopy(const DBatchProb* probs, int nprob, int64_t nmax, double* A, int from, int to, cudaStream_t st) {
   if (nprob <= 0) return;
-  bcopy_kernel<<<dim3(grid_x(nmax), nprob), kBt, 0, st>>>(probs, A, from, to);
+  launch_kernel(bcopy_kernel, dim3(grid_x(nmax), nprob), kBt, 0, st, probs, A, from, to);
 }
 
 void launch_bzero(const DBatchProb* probs, int nprob, int64_t nmax, double* A, int slot, cudaStream_t st) {
   if (nprob <= 0) return;
-  bzero_kernel<<<dim3(grid_x(nmax), nprob), kBt, 0, st>>>(probs, A, slot);
+  launch_kernel(bzero_kernel, dim3(grid_x(nmax), nprob), kBt, 0, st, probs, A, slot);
 }
 
 void launch_bmultidot(const DBatchProb* probs, int nprob, const double* A, int m, double* partial, double* out,
                       cudaStream_t st) {
   if (nprob <= 0) return;
-  bmultidot_partial_kernel<<<dim3(kBatchBlocks, nprob), kBt, 0, st>>>(probs, A, m, partial);
-  bmultidot_final_kernel<<<nprob, 128, 0, st>>>(partial, kBatchBlocks, m, out);
+  launch_kernel(bmultidot_partial_kernel, dim3(kBatchBlocks, nprob), kBt, 0, st, probs, A, m, partial);
+  launch_kernel(bmultidot_final_kernel, nprob, 128, 0, st, partial, kBatchBlocks, m, out);
 }
 
 void launch_brotate(const DBatchProb* probs, int nprob, int64_t nmax, double* A, int m, const double* R,
                     cudaStream_t st) {
   if (nprob <= 0) return;
-  brotate_kernel<<<dim3(grid_x(nmax), nprob), kBt, 0, st>>>(probs, A, m, R);
+  launch_kernel(brotate_kernel, dim3(grid_x(nmax), nprob), kBt, 0, st, probs, A, m, R);
 }
 
 void launch_bresidual(const DBatchProb* probs, int nprob, double* A, const double* eval, double* partial,
                       double* rnorm, cudaStream_t st) {
   if (nprob <= 0) return;
-  bresidual_kernel<<<dim3(kBatchBlocks, nprob), kBt, 0, st>>>(probs, A, eval, partial);
-  bsum_kernel<<<(nprob + 127) / 128, 128, 0, st>>>(partial, kBatchBlocks, nprob, rnorm);
+  launch_kernel(bresidual_kernel, dim3(kBatchBlocks, nprob), kBt, 0, st, probs, A, eval, partial);
+  launch_kernel(bsum_kernel, (nprob + 127) / 128, 128, 0, st, partial, kBatchBlocks, nprob, rnorm);
 }
 
 void launch_bprecondition(const DBatchProb* probs, int nprob, int64_t nmax, double* A, const double* eval,
                           cudaStream_t st) {
   if (nprob <= 0) return;
-  bprecondition_kernel<<<dim3(grid_x(nmax), nprob), kBt, 0, st>>>(probs, A, eval);
+  launch_kernel(bprecondition_kernel, dim3(grid_x(nmax), nprob), kBt, 0, st, probs, A, eval);
 }
 
 void launch_bproject(const DBatchProb* probs, int nprob, int64_t nmax, double* A, int rs, int t, double* partial,
                      double* sums, cudaStream_t st) {
   if (nprob <= 0) return;
-  bnorm_dot_kernel<<<dim3(kBatchBlocks, nprob), kBt, 0, st>>>(probs, A, rs, t, partial);
-  bsum_pairs_kernel<<<(nprob + 127) / 128, 128, 0, st>>>(partial, kBatchBlocks, nprob, sums);
-  bproject_kernel<<<dim3(grid_x(nmax), nprob), kBt, 0, st>>>(probs, A, rs, t, sums);
+  launch_kernel(bnorm_dot_kernel, dim3(kBatchBlocks, nprob), kBt, 0, st, probs, A, rs, t, partial);
+  launch_kernel(bsum_pairs_kernel, (nprob + 127) / 128, 128, 0, st, partial, kBatchBlocks, nprob, sums);
+  launch_kernel(bproject_kernel, dim3(grid_x(nmax), nprob), kBt, 0, st, probs, A, rs, t, sums);
 }
 
 }  // namespace mpsxx

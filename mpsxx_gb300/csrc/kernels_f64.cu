@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "kernels.hpp"
+#include "launch.hpp"
 
 namespace mpsxx {
 
@@ -503,18 +504,18 @@ void launch_gemm_f64(int transa, int transb, double alpha, const double* A, cons
                      const DTile* tiles, int ntiles, const DGemmTask* tasks, const DGemmPair* pairs,
                      double* partial, cudaStream_t st) {
   if (ntiles <= 0) return;
-  gemm_f64_kernel<<<ntiles, 256, 0, st>>>(transa, transb, alpha, A, B, C, tiles, tasks, pairs, partial);
+  launch_kernel(gemm_f64_kernel, ntiles, 256, 0, st, transa, transb, alpha, A, B, C, tiles, tasks, pairs, partial);
 }
 
 void launch_gemm_reduce(const DReduce* red, int nred, const DGemmTask* tasks, double alpha, const double* partial,
                         double* C, cudaStream_t st) {
   if (nred <= 0) return;
-  gemm_reduce_kernel<<<nred, 256, 0, st>>>(red, tasks, alpha, partial, C);
+  launch_kernel(gemm_reduce_kernel, nred, 256, 0, st, red, tasks, alpha, partial, C);
 }
 
 void launch_copy(const DCopy* tasks, int ntasks, const double* src, double* dst, int accumulate, cudaStream_t st) {
   if (ntasks <= 0) return;
-  copy_kernel<<<ntasks, 256, 0, st>>>(tasks, src, dst, accumulate);
+  launch_kernel(copy_kernel, ntasks, 256, 0, st, tasks, src, dst, accumulate);
 }
 
 void launch_scatter(const DScatterDst* dsts, int ndst, const DScatterSrc* srcs, const double* src, double* dst,
@@ -523,13 +524,13 @@ void launch_scatter(const DScatterDst* dsts, int ndst, const DScatterSrc* srcs, 
   // warps per sub-block: four waves of warps (48 on each of 152 SMs) where there are sub-blocks
   // for less, since a warp alone on a sub-block of 98 x 98 takes 40 us
   const int parts = std::min(16, std::max(1, 4 * 48 * 152 / ndst));
-  scatter_kernel<<<dim3((ndst + 7) / 8, parts), 256, 0, st>>>(dsts, ndst, srcs, src, dst);
+  launch_kernel(scatter_kernel, dim3((ndst + 7) / 8, parts), 256, 0, st, dsts, ndst, srcs, src, dst);
 }
 
 void launch_adjoint_scatter(const DScatterDst* dsts, int ndst, const DScatterSrc* srcs, const double* Y,
                             const double* src, double* g, cudaStream_t st) {
   if (ndst <= 0) return;
-  adjoint_scatter_kernel<<<ndst, 256, 0, st>>>(dsts, srcs, Y, src, g);
+  launch_kernel(adjoint_scatter_kernel, ndst, 256, 0, st, dsts, srcs, Y, src, g);
 }
 
 void launch_eig_factors(const double* G, const double* w, int d, int k, int transposed, double* out, double* xcm,
@@ -537,40 +538,40 @@ void launch_eig_factors(const double* G, const double* w, int d, int k, int tran
   const int64_t n = (int64_t)d * k;
   if (n <= 0) return;
   const int grid = static_cast<int>(std::min<int64_t>((n + 255) / 256, 4096));
-  eig_factors_kernel<<<grid, 256, 0, st>>>(G, w, d, k, transposed, out, xcm, s);
+  launch_kernel(eig_factors_kernel, grid, 256, 0, st, G, w, d, k, transposed, out, xcm, s);
 }
 
 void launch_segment_sum(const int* ptr, const int* idx, const double* g, int ne, double* G, cudaStream_t st) {
   if (ne <= 0) return;
-  segment_sum_kernel<<<(ne + 7) / 8, 256, 0, st>>>(ptr, idx, g, ne, G);
+  launch_kernel(segment_sum_kernel, (ne + 7) / 8, 256, 0, st, ptr, idx, g, ne, G);
 }
 
 void launch_diag(const DDiagTile* tiles, int ntiles, const DDiagTask* tasks, const DDiagPair* pairs, const double* L,
                  const double* R, double* out, cudaStream_t st) {
   if (ntiles <= 0) return;
   constexpr int smem = 2 * kDiagPairs * (64 + 4) * sizeof(double);  // the widest span: 4 columns by 64 rows
-  diag_kernel<<<ntiles, 256, smem, st>>>(tiles, tasks, pairs, L, R, out);
+  launch_kernel(diag_kernel, ntiles, 256, smem, st, tiles, tasks, pairs, L, R, out);
 }
 
 void launch_scal_dev(double* x, int64_t n, const double* s, int mode, cudaStream_t st) {
   if (n <= 0) return;
-  scal_dev_kernel<<<grid_for(n), 256, 0, st>>>(x, n, s, mode);
+  launch_kernel(scal_dev_kernel, grid_for(n), 256, 0, st, x, n, s, mode);
 }
 
 void launch_axpy(double* y, const double* x, int64_t n, double a, cudaStream_t st) {
   if (n <= 0) return;
-  axpy_kernel<<<grid_for(n), 256, 0, st>>>(y, x, n, a);
+  launch_kernel(axpy_kernel, grid_for(n), 256, 0, st, y, x, n, a);
 }
 
 void launch_noise_axpy(const DNoise* blocks, int nblocks, const double* seq, double noise, double* y,
                        cudaStream_t st) {
   if (nblocks <= 0) return;
-  noise_axpy_kernel<<<nblocks, 256, 0, st>>>(blocks, seq, noise, y);
+  launch_kernel(noise_axpy_kernel, nblocks, 256, 0, st, blocks, seq, noise, y);
 }
 
 void launch_copy_vec(double* y, const double* x, int64_t n, cudaStream_t st) {
   if (n <= 0) return;
-  copy_vec_kernel<<<grid_for(n), 256, 0, st>>>(y, x, n);
+  launch_kernel(copy_vec_kernel, grid_for(n), 256, 0, st, y, x, n);
 }
 
 int multidot_blocks(int64_t n) {
@@ -582,26 +583,26 @@ int multidot_blocks(int64_t n) {
 
 void launch_multidot(const double* X, int nx, const double* Y, int ny, int64_t n, int64_t stride, double* out,
                      double* partial, int nblocks, cudaStream_t st) {
-  multidot_partial_kernel<<<nblocks, 256, 0, st>>>(X, nx, Y, ny, n, stride, partial);
-  multidot_final_kernel<<<1, 128, 0, st>>>(partial, nblocks, nx * ny, out);
+  launch_kernel(multidot_partial_kernel, nblocks, 256, 0, st, X, nx, Y, ny, n, stride, partial);
+  launch_kernel(multidot_final_kernel, 1, 128, 0, st, partial, nblocks, nx * ny, out);
 }
 
 void launch_scale_blocks_rows(double* data, const int64_t* off, const int* rows, const int* cols,
                               const int64_t* s_off, int nb, const double* s, cudaStream_t st) {
   if (nb <= 0) return;
-  scale_rows_kernel<<<nb, 256, 0, st>>>(data, off, rows, cols, s_off, s);
+  launch_kernel(scale_rows_kernel, nb, 256, 0, st, data, off, rows, cols, s_off, s);
 }
 
 void launch_scale_blocks_cols(double* data, const int64_t* off, const int* rows, const int* cols,
                               const int64_t* s_off, int nb, const double* s, cudaStream_t st) {
   if (nb <= 0) return;
-  scale_cols_kernel<<<nb, 256, 0, st>>>(data, off, rows, cols, s_off, s);
+  launch_kernel(scale_cols_kernel, nb, 256, 0, st, data, off, rows, cols, s_off, s);
 }
 
 void launch_transpose(const double* src, double* dst, int rows, int cols, cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return;
   dim3 grid((cols + 31) / 32, (rows + 31) / 32);
-  transpose_kernel<<<grid, dim3(32, 8), 0, st>>>(src, dst, rows, cols);
+  launch_kernel(transpose_kernel, grid, dim3(32, 8), 0, st, src, dst, rows, cols);
 }
 
 }  // namespace mpsxx

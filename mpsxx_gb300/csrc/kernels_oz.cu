@@ -626,11 +626,7 @@ __global__ void __launch_bounds__(256, 4) oz_pack_kernel(const OzPackJobs jobs) 
 
 void launch_gemm_oz(const OzGemmArgs& a, cudaStream_t st) {
   if (a.nctas <= 0) return;
-  static bool ready = false;
-  if (!ready) {
-    cudaFuncSetAttribute(gemm_oz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    ready = true;
-  }
+  allow_smem<gemm_oz_kernel>(SMEM_BYTES);
   launch_chained(gemm_oz_kernel, dim3(a.nctas), NTHREADS, SMEM_BYTES, st, a);
 }
 

@@ -577,22 +577,18 @@ void launch_gemm_pk(const uint8_t* Apk, const uint8_t* Bpk, double alpha, double
                     int out_packed, int single, int* err, cudaStream_t st, uint64_t timeout_ns,
                     const int64_t* row_map, bool chained) {
   if (ntiles <= 0) return;
-  static int nsm = 0;
-  if (nsm == 0) {
-    cudaFuncSetAttribute(gemm_pk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (nsm <= 0) nsm = 152;
-  }
+  allow_smem<gemm_pk_kernel>(SMEM_BYTES);
+  int dev = 0, nsm = 0;
+  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+  cuda_check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev), "multiprocessor count");
   // one persistent CTA per SM; the bound covers the whole launch, not one tile
   const int grid = ntiles < nsm ? ntiles : nsm;
   if (chained)
     launch_chained(gemm_pk_kernel, dim3(grid), NTHREADS, SMEM_BYTES, st, Apk, Bpk, alpha, C, Cpk, tiles, ntiles, tasks,
                    pairs, partial, out_packed, single, err, timeout_ns, row_map);
   else
-    gemm_pk_kernel<<<grid, NTHREADS, SMEM_BYTES, st>>>(Apk, Bpk, alpha, C, Cpk, tiles, ntiles, tasks, pairs, partial,
-                                                       out_packed, single, err, timeout_ns, row_map);
+    launch_kernel(gemm_pk_kernel, grid, NTHREADS, SMEM_BYTES, st, Apk, Bpk, alpha, C, Cpk, tiles, ntiles, tasks, pairs,
+                  partial, out_packed, single, err, timeout_ns, row_map);
 }
 
 void launch_pack(const DPack* packs, int npacks, const double* src, uint8_t* dst, cudaStream_t st, bool chained) {
@@ -600,7 +596,7 @@ void launch_pack(const DPack* packs, int npacks, const double* src, uint8_t* dst
   if (chained)
     launch_chained(pack_kernel, dim3(npacks), 256, 0, st, packs, src, dst);
   else
-    pack_kernel<<<npacks, 256, 0, st>>>(packs, src, dst);
+    launch_kernel(pack_kernel, npacks, 256, 0, st, packs, src, dst);
 }
 
 void launch_gemm_pk_reduce(const DReduce* red, int nred, const DGemmTask* tasks, double alpha, const double* partial,
@@ -610,7 +606,7 @@ void launch_gemm_pk_reduce(const DReduce* red, int nred, const DGemmTask* tasks,
   if (chained)
     launch_chained(gemm_pk_reduce_kernel, grid, 256, 0, st, red, tasks, alpha, partial, C);
   else
-    gemm_pk_reduce_kernel<<<grid, 256, 0, st>>>(red, tasks, alpha, partial, C);
+    launch_kernel(gemm_pk_reduce_kernel, grid, 256, 0, st, red, tasks, alpha, partial, C);
 }
 
 }  // namespace mpsxx

@@ -22,6 +22,7 @@
 #include <cstdint>
 
 #include "kernels.hpp"
+#include "launch.hpp"
 
 namespace mpsxx {
 namespace {
@@ -241,12 +242,12 @@ __global__ void eig_factors_batched_kernel(const DEigBlock* __restrict__ blocks,
 
 void launch_gram_pad(const DEigBlock* blocks, int nblocks, double* G, cudaStream_t st) {
   if (nblocks <= 0) return;
-  gram_pad_kernel<<<nblocks, 128, 0, st>>>(blocks, G);
+  launch_kernel(gram_pad_kernel, nblocks, 128, 0, st, blocks, G);
 }
 
 void launch_eig_factors_batched(const DEigBlock* blocks, int nblocks, const double* G, cudaStream_t st) {
   if (nblocks <= 0) return;
-  eig_factors_batched_kernel<<<nblocks, 256, 0, st>>>(blocks, G);
+  launch_kernel(eig_factors_batched_kernel, nblocks, 256, 0, st, blocks, G);
 }
 
 size_t jacobi_svd_smem(int m, int n) {
@@ -257,12 +258,8 @@ size_t jacobi_svd_smem(int m, int n) {
 void launch_jacobi_svd(const DSvdBlock* blocks, int nblocks, size_t smem_bytes, double* out, int* info,
                        cudaStream_t st) {
   if (nblocks <= 0) return;
-  static size_t configured = 0;
-  if (smem_bytes > configured) {
-    cudaFuncSetAttribute(jacobi_svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes));
-    configured = smem_bytes;
-  }
-  jacobi_svd_kernel<<<nblocks, kJt, smem_bytes, st>>>(blocks, out, info);
+  allow_smem<jacobi_svd_kernel>(smem_bytes);
+  launch_kernel(jacobi_svd_kernel, nblocks, kJt, smem_bytes, st, blocks, out, info);
 }
 
 }  // namespace mpsxx

@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <exception>
 #include <mutex>
 #include <string>
 
@@ -84,8 +85,10 @@ extern "C" int mpsxx_multidot_noalloc(const double* X, int nx, const double* Y, 
   }
   const int nblocks = mpsxx::multidot_blocks(n);
   if (nblocks > kMaxBlocks) return fail(MPSXX_INVALID_ARGUMENT, "mpsxx_multidot_noalloc: scratch too small");
-  mpsxx::launch_multidot(X, nx, Y, ny, n, stride, out, scratch, nblocks, static_cast<cudaStream_t>(stream));
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return fail(MPSXX_CUDA, "mpsxx_multidot_noalloc: kernel launch failed");
+  try {
+    mpsxx::launch_multidot(X, nx, Y, ny, n, stride, out, scratch, nblocks, static_cast<cudaStream_t>(stream));
+  } catch (const std::exception&) {
+    return fail(MPSXX_CUDA, "mpsxx_multidot_noalloc: kernel launch failed");
+  }
   return MPSXX_OK;
 }

@@ -15,6 +15,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -31,6 +32,7 @@ std::map<void*, size_t> blocks;
 std::map<const void*, std::string> names;
 std::map<std::pair<int, const void*>, int> smem;
 std::string fail_name, text;
+std::set<cudaStream_t> capturing;
 
 struct Config {
   dim3 grid, block;
@@ -163,6 +165,20 @@ cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
   *ms = 1.0f;
   return cudaSuccess;
 }
+cudaError_t cudaStreamBeginCapture(cudaStream_t st, cudaStreamCaptureMode) {
+  return capturing.insert(st).second ? cudaSuccess : result(cudaErrorIllegalState);
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t st, cudaGraph_t* g) {
+  *g = reinterpret_cast<cudaGraph_t>(16);
+  return capturing.erase(st) ? cudaSuccess : result(cudaErrorIllegalState);
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
+  *e = reinterpret_cast<cudaGraphExec_t>(16);
+  return cudaSuccess;
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   std::lock_guard<std::recursive_mutex> lk(mu);
   if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) smem[{device, f}] = v;

@@ -18,3 +18,61 @@ def test_wavefunctions_that_do_not_stack_take_the_general_path(dims, cols, qrow)
     out = [error(core.compute_sigma_vector, ctx, L, R, P, P.like()), len(launches("gemm_f64"))]
     """)
     assert out == [0, 2]
+
+
+def test_products_on_a_second_device():
+    """Limits of shared memory that are raised for a kernel hold on one device only."""
+    out = run("""
+    fake.fake_devices(2)
+    out = []
+    for dev in (0, 1):
+        ctx = core.Context(dev)
+        ctx.set_fp64_route(0.0)
+        L, R, P = operands(core, ctx)
+        launches()
+        for prec in (core.FP64, core.SPLIT_TF32):
+            core.set_precision(ctx, prec)
+            core.compute_sigma_vector(ctx, L, R, P, P.like())
+        out.append(sorted({x.split()[1] for x in launches("%d " % dev)}))
+    """)
+    assert out[0] == out[1]
+    assert any("gemm_oz_kernel" in x for x in out[1]) and any("gemm_pk_kernel" in x for x in out[1])
+
+
+@pytest.mark.parametrize("kernel", ["gemm_oz", "oz_pack", "gemm_f64", "gemm_pk_kernel", "pack_kernel", "diag_kernel"])
+def test_a_launch_that_fails_is_an_error(kernel):
+    """Once the kernel can be launched the same calls succeed."""
+    out = run(f"""
+    ctx = core.Context(0)
+    L, R, P = operands(core, ctx)
+    def calls():
+        bad = []
+        for prec, route in ((core.FP64, 0.0), (core.FP64, float("inf")), (core.SPLIT_TF32, 0.0)):
+            core.set_precision(ctx, prec)
+            ctx.set_fp64_route(route)
+            bad.append(error(core.compute_sigma_vector, ctx, L, R, P, P.like()))
+        bad.append(error(core.compute_diagonal_elements, ctx, L, R, P.like()))
+        return bad
+    fake.fake_fail_launch({kernel!r}.encode())
+    out = [calls()]
+    fake.fake_fail_launch(b"")
+    out.append(calls())
+    """)
+    assert 6 in out[0] and set(out[0]) <= {0, 6}
+    assert out[1] == [0, 0, 0, 0]
+
+
+def test_a_launch_that_fails_while_a_graph_is_captured():
+    """The capture ends with the call; the next call captures again."""
+    out = run("""
+    ctx = core.Context(0)
+    core.set_precision(ctx, core.SPLIT_TF32)
+    ctx.set_sigma_schedule(1)
+    L, R, P = operands(core, ctx, dims=(40, 24, 30))
+    fake.fake_fail_launch(b"gemm_pk_kernel")
+    out = [error(core.compute_sigma_vector, ctx, L, R, P, P.like())]
+    fake.fake_fail_launch(b"")
+    out.append(error(core.compute_sigma_vector, ctx, L, R, P, P.like()))
+    out.append(len(launches("gemm_pk_kernel")))
+    """)
+    assert out[:2] == [6, 0] and out[2] > 2  # a pair of products for each group of w
