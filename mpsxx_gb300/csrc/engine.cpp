@@ -1378,29 +1378,34 @@ static void sigma_run_pk_whole(Context& ctx, SigmaPlan& p, double* sigma) {
 static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTensor& R, const double* psi,
                          double* sigma) {
   if (!p.stacks) return false;
-  std::vector<OzSource> pack;
+  std::vector<std::pair<OzOperand*, const DTensor*>> stale;
   {
     PhaseTimer tm(ctx, kPhSigmaPlan);
-    if (!p.o1.built) build_oz_gemm(ctx, p.o1, p.s1, L, p.psi_layout, true);
-    if (!p.o2.built) build_oz_gemm(ctx, p.o2, p.s2, p.scr1, R, false, &p.o1, &p.s1);
-    if (!oz_reserve(ctx, {&p.o1, &p.o2})) return false;
+    const bool room = oz_reserve(ctx, {&p.o1, &p.o2}, [&] {
+      if (!p.o1.built) build_oz_gemm(ctx, p.o1, p.s1, L, p.psi_layout, true);
+      if (!p.o2.built) build_oz_gemm(ctx, p.o2, p.s2, p.scr1, R, false, &p.o1, &p.s1);
+      return OzScratch{&ctx.scr1, p.o1.tiled_elems * sizeof(double)};
+    });
+    if (!room) return false;
     for (auto& x : {std::make_pair(&p.o1.a, &L), std::make_pair(&p.o2.b, &R)}) {
-      OzOperand& o = *x.first;
-      if (o.src_layout == x.second->layout_id && o.src_version == x.second->data_version &&
-          (!x.second->exposed || o.src_call == ctx.call))
-        continue;
-      pack.push_back(OzSource{&o, x.second->d});
-      o.src_layout = x.second->layout_id;
-      o.src_version = x.second->data_version;
-      o.src_call = ctx.call;
+      const OzOperand& o = *x.first;
+      if (o.src_layout != x.second->layout_id || o.src_version != x.second->data_version ||
+          (x.second->exposed && o.src_call != ctx.call))
+        stale.push_back(x);
     }
     tm.stop();
     ctx.timers[kPhSigma] -= tm.dt;  // counted as planning, not as H_eff * psi
   }
-  ctx.scr1.ensure(std::max<int64_t>(p.o1.tiled_elems, 1) * sizeof(double), ctx.stream);
   double* scr = ctx.scr1.as<double>();
+  std::vector<OzSource> pack;
+  for (const auto& x : stale) pack.push_back(OzSource{x.first, x.second->d});
   pack.push_back(OzSource{&p.o1.b, psi});
   oz_pack(ctx, pack);
+  for (const auto& x : stale) {  // (queued: the operands hold these data from here on)
+    x.first->src_layout = x.second->layout_id;
+    x.first->src_version = x.second->data_version;
+    x.first->src_call = ctx.call;
+  }
   run_oz_gemm(ctx, p.o1, p.s1, 1.0, L.d, psi, scr, true);
   oz_pack(ctx, {{&p.o2.a, scr}});
   run_oz_gemm(ctx, p.o2, p.s2, 1.0, scr, R.d, sigma, false);
@@ -1726,9 +1731,12 @@ RenormPlan& renorm_plan(Context& ctx, bool forward, const Tensor& opr0, const Te
 // digits go back to the block cache afterwards.  False: no memory for it.
 static bool renorm_run_oz(Context& ctx, RenormPlan& rp, const DTensor& bra, const DTensor& opr0, const DTensor& ket,
                           double* scr, double* out) {
-  if (!rp.o1.built) build_oz_gemm(ctx, rp.o1, rp.p1, conj_view(bra), opr0);
-  if (!rp.o2.built) build_oz_gemm(ctx, rp.o2, rp.p2, rp.scr, ket);
-  if (!oz_reserve(ctx, {&rp.o1, &rp.o2})) return false;
+  const bool room = oz_reserve(ctx, {&rp.o1, &rp.o2}, [&] {
+    if (!rp.o1.built) build_oz_gemm(ctx, rp.o1, rp.p1, conj_view(bra), opr0);
+    if (!rp.o2.built) build_oz_gemm(ctx, rp.o2, rp.p2, rp.scr, ket);
+    return OzScratch{};
+  });
+  if (!room) return false;
   oz_pack(ctx, {{&rp.o1.a, rp.o1.swap ? opr0.d : bra.d},
                 {&rp.o1.b, rp.o1.swap ? bra.d : opr0.d},
                 {rp.o2.swap ? &rp.o2.a : &rp.o2.b, ket.d}});

@@ -292,8 +292,19 @@ struct OzGemm {
   int64_t tiled_elems = 0;
   DevView<DOzTiled> pairs_tiled;
   size_t partial_bytes() const { return size_t(nslots) * kOzTileM * kOzTileN * sizeof(double); }
-  int64_t device_bytes() const { return a.bytes + b.bytes + 4 * (int64_t(a.rows) + b.rows); }
-  bool held() const { return a.buf.p && b.buf.p; }
+  void clear() {  // what a build that did not end has left
+    for (OzOperand* o : {&a, &b}) {
+      o->h_packs.clear();
+      o->h_segs.clear();
+      o->bytes = 0;
+      o->rows = 0;
+    }
+    h_tiles.clear();
+    h_reduce.clear();
+    task_place.clear();
+    tiled_elems = 0;
+    nslots = 0;
+  }
   void release() {
     a.release();
     b.release();
@@ -312,9 +323,14 @@ void oz_pack(Context& ctx, const std::vector<OzSource>& what);
 // C = (assign) or += alpha op(A) op(B) from the packed operands.
 void run_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, double alpha, const double* A, const double* B, double* C,
                  bool assign);
-// Device memory for the plans' packed operands: false (nothing held) when it would take
-// more than half of what is free.
-bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs);
+// Device memory of a product's plans, which `build` makes where they are not built: their
+// packed operands, split-K slots and the scratch that it returns.  False where that would
+// take more than half of what is free, or where an allocation fails (nothing is held then).
+struct OzScratch {
+  DevBuf* buf = nullptr;
+  size_t bytes = 0;
+};
+bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs, const std::function<OzScratch()>& build);
 // whether a plan of that many FLOPs runs on the tensor cores
 bool oz_wanted(const Context& ctx, double flops);
 // Output tiles of every task with long pair lists split along K (engine.cpp)

@@ -83,6 +83,7 @@ void pack_blocks(OzOperand& o, const Tensor& t, const std::vector<View>& view, b
 
 void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a, const Tensor& b, bool tiled_out,
                    const OzGemm* from, const GemmPlan* from_plan) {
+  og.clear();
   // operand blocks as rows x K
   std::vector<View> va(a.tags.size()), vb(b.tags.size());
   std::set<int32_t> used_a, used_b;
@@ -247,21 +248,29 @@ bool oz_wanted(const Context& ctx, double flops) {
   return flops >= (ctx.oz_min_flops >= 0.0 ? ctx.oz_min_flops : kOzMinFlops);
 }
 
-bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs) {
-  int64_t need = 0;
-  for (OzGemm* g : gs)
-    if (!g->held()) need += g->device_bytes();
-  if (need > kOzSmallBytes) {
-    size_t free_b = 0, total_b = 0;
-    cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-    if (need > static_cast<int64_t>((free_b + block_cache_bytes()) / 2)) return false;
-  }
+bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs, const std::function<OzScratch()>& build) {
   try {
-    for (OzGemm* g : gs)
+    const OzScratch scratch = build();
+    std::vector<std::pair<DevBuf*, size_t>> bufs;
+    size_t part = 16;
+    for (OzGemm* g : gs) {
       for (OzOperand* o : {&g->a, &g->b}) {
-        o->buf.ensure(std::max<int64_t>(o->bytes, 16), ctx.stream);
-        o->exps.ensure(size_t(std::max(o->rows, 1)) * sizeof(int), ctx.stream);
+        bufs.push_back({&o->buf, std::max<int64_t>(o->bytes, 16)});
+        bufs.push_back({&o->exps, size_t(std::max(o->rows, 1)) * sizeof(int)});
       }
+      part = std::max(part, g->partial_bytes());
+    }
+    bufs.push_back({&ctx.gemm_part, part});
+    if (scratch.buf) bufs.push_back({scratch.buf, std::max<size_t>(scratch.bytes, 16)});
+    int64_t need = 0;
+    for (const auto& b : bufs)
+      if (b.first->cap < b.second) need += static_cast<int64_t>(b.second);
+    if (need > kOzSmallBytes) {
+      size_t free_b = 0, total_b = 0;
+      cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+      if (need > static_cast<int64_t>((free_b + block_cache_bytes()) / 2)) return false;
+    }
+    for (const auto& b : bufs) b.first->ensure(b.second, ctx.stream);
   } catch (const Error& e) {
     if (e.code != kAlloc) throw;
     for (OzGemm* g : gs) g->release();
@@ -275,17 +284,16 @@ void oz_pack(Context& ctx, const std::vector<OzSource>& what) {
   OzPackJobs jobs{};
   for (const OzSource& w : what) {
     OzOperand& o = *w.o;
-    ++o.seq;
     jobs.job[jobs.n++] = OzPackJob{o.packs.get(), o.segs.get(), w.src, o.buf.as<uint8_t>(), o.exps.as<int>(),
-                                   o.flag.get(), static_cast<int>(o.h_packs.size()), o.seq};
+                                   o.flag.get(), static_cast<int>(o.h_packs.size()), o.seq + 1};
   }
   launch_oz_pack(jobs, ctx.stream);
+  for (const OzSource& w : what) ++w.o->seq;
   ctx.kernel_launches += 1;
 }
 
 void run_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, double alpha, const double* A, const double* B, double* C,
                  bool assign) {
-  ctx.gemm_part.ensure(std::max<size_t>(og.partial_bytes(), 16), ctx.stream);
   OzGemmArgs a{};
   a.Apk = og.a.buf.as<uint8_t>();
   a.Bpk = og.b.buf.as<uint8_t>();

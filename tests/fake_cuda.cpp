@@ -3,7 +3,7 @@
 // A test asks for the failures of interest:
 //   fake_devices(n)         n devices; what is set for one device does not hold on another
 //   fake_limit(bytes)       allocations beyond that many bytes in all fail (0: none does)
-//   fake_fail_alloc(bytes)  the next allocation of at least that size fails (0: none does)
+//   fake_fail_alloc(k, n)   after k more allocations, n fail
 //   fake_fail_launch(name)  launches of kernels whose name contains it fail ("": none does)
 //   fake_log(buf, n)        the launches since the last call, one "device kernel note" a line
 // A launch with more than 48 KB of dynamic shared memory fails, as on a device, unless the
@@ -26,7 +26,8 @@ std::recursive_mutex mu;
 thread_local int device = 0;
 thread_local cudaError_t last = cudaSuccess;
 int ndevices = 1;
-size_t limit = 0, fail_bytes = 0, used = 0;
+size_t limit = 0, used = 0;
+int fail_after = 0, fail_count = 0;
 constexpr size_t kTotal = size_t(64) << 30;
 std::map<void*, size_t> blocks;
 std::map<const void*, std::string> names;
@@ -65,7 +66,10 @@ cudaError_t launch(const void* f, size_t shared, void** args) {
 extern "C" {
 void fake_devices(int n) { ndevices = n; }
 void fake_limit(size_t b) { limit = b; }
-void fake_fail_alloc(size_t b) { fail_bytes = b; }
+void fake_fail_alloc(int k, int n) {
+  fail_after = k;
+  fail_count = n;
+}
 void fake_fail_launch(const char* n) { fail_name = n; }
 size_t fake_used() { return used; }
 int fake_log(char* buf, int n) {
@@ -104,8 +108,10 @@ cudaError_t cudaPeekAtLastError() { return last; }
 const char* cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "invalid"; }
 cudaError_t cudaMalloc(void** p, size_t n) {
   std::lock_guard<std::recursive_mutex> lk(mu);
-  if (fail_bytes && n >= fail_bytes) {
-    fail_bytes = 0;
+  if (fail_after > 0) {
+    --fail_after;
+  } else if (fail_count > 0) {
+    --fail_count;
     return result(cudaErrorMemoryAllocation);
   }
   if (used + n > kTotal || (limit && used + n > limit)) return result(cudaErrorMemoryAllocation);

@@ -21,8 +21,7 @@ from mpsxx_gb300 import core
 from mpsxx_gb300._lib import MpsxxError
 from tests.fakecuda import operands
 fake = ctypes.CDLL({fake!r})
-for f in ("fake_limit", "fake_fail_alloc"):
-    getattr(fake, f).argtypes = [ctypes.c_size_t]
+fake.fake_limit.argtypes = [ctypes.c_size_t]
 fake.fake_used.restype = ctypes.c_size_t
 
 def launches(name=""):
@@ -30,6 +29,11 @@ def launches(name=""):
     b = ctypes.create_string_buffer(n)
     fake.fake_log(b, n)
     return [x for x in b.value.decode().split("\\n") if x and name in x]
+
+def empty_cache(ctx):
+    fake.fake_fail_alloc(0, 2)
+    assert error(core.Tensor.create, ctx, (0, 0), [[(0, 0)]], [[1 << 28]]) == 2
+    fake.fake_fail_alloc(0, 0)
 
 def error(f, *a):
     try:

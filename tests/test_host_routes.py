@@ -76,3 +76,36 @@ def test_a_launch_that_fails_while_a_graph_is_captured():
     out.append(len(launches("gemm_pk_kernel")))
     """)
     assert out[:2] == [6, 0] and out[2] > 2  # a pair of products for each group of w
+
+
+def test_products_after_an_allocation_that_failed():
+    """Whichever allocation of a sliced product fails, the call gives a result on the FP64 pipe or
+    an allocation error, and the next one cuts the digits that the first did not."""
+    out = run("""
+    out = []
+    for k in range(40):
+        L = R = P = S = ctx = None
+        ctx = core.Context(0)
+        ctx.set_fp64_route(0.0)
+        empty_cache(ctx)
+        L, R, P = operands(core, ctx, (300, 200), cols=(40, 300))
+        S = P.like()
+        launches()
+        fake.fake_fail_alloc(k, 2)  # (an allocation is tried again after the cache is emptied)
+        code = error(core.compute_sigma_vector, ctx, L, R, P, S)
+        fake.fake_fail_alloc(0, 0)
+        a = [x.split(None, 1)[1] for x in launches()]
+        code2 = error(core.compute_sigma_vector, ctx, L, R, P, S)
+        b = [x.split(None, 1)[1] for x in launches()]
+        digits = lambda x: [int(y.split()[1]) for y in x if "oz_pack" in y]
+        pipe = sum("gemm_f64" in y for y in a)
+        out.append([code, pipe, digits(a), code2, digits(b)])
+    """)
+    failed = [x for x in out if x[0] or x[1]]
+    assert len(failed) > 4 and any(x[1] for x in failed) and out[-1][:2] == [0, 0]
+    for code, pipe, first, code2, second in out:
+        assert code in (0, 2) and code2 == 0
+        if code == 0:
+            assert (pipe, first) in ((2, []), (0, [3, 1]))
+        # L, R and psi; psi alone where L's and R's digits are there
+        assert second == ([1, 1] if 3 in first else [3, 1])
