@@ -226,6 +226,25 @@ void build_gemm_plan(GemmPlan& plan, Trans ta, Trans tb, const Tensor& a, const 
                      int K, std::vector<GemmTaskRef>&& tasks);
 
 // Blocks of one tensor packed as split-TF32 tensor-core tiles (one role: A or B).
+// Whose data a packed copy holds.
+struct PackedSource {
+  uint64_t layout = 0, version = ~0ull, call = 0;
+  bool printed = false;  // print: fingerprint of the data
+  Fingerprint print{};
+  // whether the copy is t's data as they are in call number `now` (Context::call)
+  bool is(const DTensor& t, uint64_t now) const {
+    return same(t) && (!t.exposed || call == now);
+  }
+  bool same(const DTensor& t) const { return layout == t.layout_id && version == t.data_version; }
+  void set(const DTensor& t, uint64_t now) {
+    layout = t.layout_id;
+    version = t.data_version;
+    call = now;
+    printed = false;
+  }
+  void reset() { *this = PackedSource{}; }
+};
+
 struct Packed {
   DevBuf buf;
   std::vector<int64_t> base;  // per block slot: byte offset of its tile grid (-1: not packed)
@@ -233,7 +252,7 @@ struct Packed {
   std::vector<DPack> h_packs;
   DevArray<DPack> packs;
   int64_t bytes = 0;
-  uint64_t src_layout = 0, src_version = ~0ull;  // what the buffer currently holds
+  PackedSource src;  // what the buffer currently holds
 };
 
 // Split-TF32 execution of one GemmPlan: the operand blocks the plan touches are
@@ -258,12 +277,11 @@ struct OzOperand {
   int64_t bytes = 0;
   int rows = 0;
   int seq = 0;  // packings so far
-  uint64_t src_layout = 0, src_version = ~0ull, src_call = 0;  // what the digits are of
+  PackedSource src;  // what the digits are of
   void release() {
     buf.release();
     exps.release();
-    src_layout = 0;
-    src_version = ~0ull;
+    src.reset();
   }
 };
 
@@ -500,6 +518,7 @@ struct Context {
   DevBuf partial;    // reduction partials
   DevBuf scalars;    // small device scalars
   DevBuf dv_sums;    // Davidson: ticket, sums and partials of the fused vector kernels
+  DevBuf print_sums; // fingerprints: sums and counts of CTAs
   cudaEvent_t dv_done = nullptr;
   DevBuf svd_work;   // solver workspace
   DevBuf svd_mats;   // per-block SVD matrices
@@ -620,6 +639,7 @@ void compute_sigma_vector(Context& ctx, const DTensor& L, const DTensor& R, cons
 int* device_err_flag(Context& ctx);
 void release_err_flag(Context& ctx);
 double* device_host_sums(Context& ctx, double** host);
+Fingerprint* device_host_prints(Context& ctx, volatile Fingerprint** host);
 void check_device_error(Context& ctx);
 
 // average device seconds of `reps` sigma applications (CUDA events on ctx.stream)

@@ -173,6 +173,18 @@ void launch_gemm_pk_reduce(const DReduce* red, int nred, const DGemmTask* tasks,
 void launch_pack(const DPack* packs, int npacks, const double* src, uint8_t* dst, cudaStream_t st,
                  bool chained = false);
 int pk_smem_bytes();
+// 128-bit fingerprints of up to two arrays into mapped host memory; sums: kPrintWords zeroed
+// words on the device, zero again after the launch.
+struct Fingerprint {
+  unsigned long long h[2];
+};
+struct PrintJobs {
+  const double* x[2];
+  int64_t n[2];
+  Fingerprint* out[2];
+};
+constexpr int kPrintWords = 6;
+void launch_fingerprints(const PrintJobs& jobs, int njobs, unsigned long long* sums, cudaStream_t st);
 
 // ---- FP64 GEMM on the tensor cores (kernels_oz.cu) ------------------------------
 // Packed digit tiles: A operands in 128-row tiles (a last tile of its rows rounded up to 8:

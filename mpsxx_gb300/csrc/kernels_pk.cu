@@ -529,6 +529,64 @@ __global__ void __launch_bounds__(256) pack_kernel(const DPack* __restrict__ pac
   }
 }
 
+// Fingerprints of arrays (blockIdx.y): 128-bit sums of products (x_i + k_i) (x_j + k_j) over
+// pairs of elements, taken as integers, with keys that depend on their places (NH: Black,
+// Halevi, Krawczyk, Krovetz, Rogaway 1999, "UMAC", for 64-bit words; the keys are multiples of
+// 2^64 over the golden ratio).  Arrays that differ have equal sums with a chance of about
+// 2^-64.  The order of addition is free, but pairs and CTAs are the same for equal sizes.  The
+// kernel is bound by the reading of the arrays (2.45 GB in 0.37 ms): 10 instructions an element
+// on the integer pipe.
+__global__ void __launch_bounds__(256) fingerprint_kernel(const PrintJobs jobs, unsigned long long* sums) {
+  using u64 = unsigned long long;
+  __shared__ u64 part[2][8];
+  const u64* __restrict__ x = reinterpret_cast<const u64*>(jobs.x[blockIdx.y]);
+  const int64_t n = jobs.n[blockIdx.y], step = (int64_t)gridDim.x * 256;
+  constexpr u64 kKey = 0x9e3779b97f4a7c15ull;
+  unsigned __int128 acc = 0;
+  int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x;
+  u64 key = (u64)(i + 1) * kKey;  // of element i
+  const u64 kstep = (u64)step * kKey;
+  auto add = [&](u64 v, u64 w) {  // elements i, i + step
+    acc += (unsigned __int128)(v + key) * (w + key + kstep);
+    key += 2 * kstep;
+  };
+  constexpr int U = 8;
+  for (; i + (U - 1) * step < n; i += U * step) {
+    u64 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = x[i + u * step];
+#pragma unroll
+    for (int u = 0; u < U; u += 2) add(v[u], v[u + 1]);
+  }
+  for (; i < n; i += 2 * step) add(x[i], i + step < n ? x[i + step] : 0);
+  u64 a = (u64)acc, b = (u64)(acc >> 64);
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    part[0][threadIdx.x >> 5] = a;
+    part[1][threadIdx.x >> 5] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < 8; ++w) {
+    a += part[0][w];
+    b += part[1][w];
+  }
+  unsigned long long* s = sums + 3 * blockIdx.y;  // two sums and the count of CTAs
+  atomicAdd(s, a);
+  atomicAdd(s + 1, b);
+  __threadfence();
+  if (atomicAdd(s + 2, 1ull) != gridDim.x - 1) return;
+  __threadfence();
+  volatile Fingerprint* out = jobs.out[blockIdx.y];
+  out->h[0] = atomicExch(s, 0ull);
+  out->h[1] = atomicExch(s + 1, 0ull);
+  s[2] = 0;
+  __threadfence_system();
+}
+
 // Split-K partials of one output tile summed into C: one thread per row and pair of columns
 // of the tile's valid part (tail tiles are mostly padding; threads past it exit at once).  A
 // slot holds column pairs, each over all rows, so that both the GEMM's stores (a row per lane)
@@ -597,6 +655,14 @@ void launch_pack(const DPack* packs, int npacks, const double* src, uint8_t* dst
     launch_chained(pack_kernel, dim3(npacks), 256, 0, st, packs, src, dst);
   else
     launch_kernel(pack_kernel, npacks, 256, 0, st, packs, src, dst);
+}
+
+void launch_fingerprints(const PrintJobs& jobs, int njobs, unsigned long long* sums, cudaStream_t st) {
+  int64_t n = 1;
+  for (int j = 0; j < njobs; ++j) n = n < jobs.n[j] ? jobs.n[j] : n;
+  // two elements a thread at least, eight CTAs an SM at most
+  const int64_t want = (n + 511) / 512;
+  launch_kernel(fingerprint_kernel, dim3(want < 152 * 8 ? want : 152 * 8, njobs), 256, 0, st, jobs, sums);
 }
 
 void launch_gemm_pk_reduce(const DReduce* red, int nred, const DGemmTask* tasks, double alpha, const double* partial,

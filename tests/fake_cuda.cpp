@@ -5,6 +5,7 @@
 //   fake_limit(bytes)       allocations beyond that many bytes in all fail (0: none does)
 //   fake_fail_alloc(k, n)   after k more allocations, n fail
 //   fake_fail_launch(name)  launches of kernels whose name contains it fail ("": none does)
+//   fake_contents(v)        what fingerprints say of every array from here on
 //   fake_log(buf, n)        the launches since the last call, one "device kernel note" a line
 // A launch with more than 48 KB of dynamic shared memory fails, as on a device, unless the
 // kernel's limit was raised on the current one.
@@ -28,6 +29,7 @@ thread_local cudaError_t last = cudaSuccess;
 int ndevices = 1;
 size_t limit = 0, used = 0;
 int fail_after = 0, fail_count = 0;
+unsigned long long contents = 1;
 constexpr size_t kTotal = size_t(64) << 30;
 std::map<void*, size_t> blocks;
 std::map<const void*, std::string> names;
@@ -47,7 +49,7 @@ cudaError_t result(cudaError_t e) {
   return e;
 }
 
-cudaError_t launch(const void* f, size_t shared, void** args) {
+cudaError_t launch(const void* f, dim3 grid, size_t shared, void** args) {
   std::lock_guard<std::recursive_mutex> lk(mu);
   const std::string& n = names[f];
   if (!fail_name.empty() && n.find(fail_name) != std::string::npos) return result(cudaErrorInvalidValue);
@@ -57,6 +59,10 @@ cudaError_t launch(const void* f, size_t shared, void** args) {
   if (n.find("oz_pack_kernel") != std::string::npos) {
     const auto* j = static_cast<const mpsxx::OzPackJobs*>(args[0]);
     text += " " + std::to_string(j->n);
+  }
+  if (n.find("fingerprint_kernel") != std::string::npos) {
+    const auto* j = static_cast<const mpsxx::PrintJobs*>(args[0]);
+    for (unsigned i = 0; i < grid.y; ++i) j->out[i]->h[0] = j->out[i]->h[1] = contents;
   }
   text += "\n";
   return cudaSuccess;
@@ -71,6 +77,7 @@ void fake_fail_alloc(int k, int n) {
   fail_count = n;
 }
 void fake_fail_launch(const char* n) { fail_name = n; }
+void fake_contents(unsigned long long v) { contents = v; }
 size_t fake_used() { return used; }
 int fake_log(char* buf, int n) {
   std::lock_guard<std::recursive_mutex> lk(mu);
@@ -191,7 +198,7 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
-  return launch(f, c->dynamicSmemBytes, args);
+  return launch(f, c->gridDim, c->dynamicSmemBytes, args);
 }
 
 // what the compiler's launch syntax and module registration call
@@ -223,8 +230,8 @@ cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* f) {
   *k = reinterpret_cast<cudaKernel_t>(const_cast<void*>(f));
   return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void** args, size_t s, cudaStream_t) {
-  return launch(reinterpret_cast<const void*>(k), s, args);
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3, void** args, size_t s, cudaStream_t) {
+  return launch(reinterpret_cast<const void*>(k), grid, s, args);
 }
 
 int cusolverDnCreate(void** h) {

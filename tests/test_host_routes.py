@@ -109,3 +109,31 @@ def test_products_after_an_allocation_that_failed():
             assert (pipe, first) in ((2, []), (0, [3, 1]))
         # L, R and psi; psi alone where L's and R's digits are there
         assert second == ([1, 1] if 3 in first else [3, 1])
+
+
+@pytest.mark.parametrize("precision, kernel", [("FP64", "oz_pack_kernel"), ("SPLIT_TF32", "pack_kernelEPKNS_5DPack")])
+def test_operators_are_packed_anew_where_a_caller_may_have_written_them(precision, kernel):
+    """Packed operators are kept between products.  Of a tensor whose device pointer was handed
+    out the data may be other data in every call: digits are cut anew, split operators packed
+    anew where their fingerprint is another one (or none was taken of the packed data)."""
+    out = run(f"""
+    ctx = core.Context(0)
+    core.set_precision(ctx, core.{precision})
+    ctx.set_fp64_route(0.0)
+    ctx.set_sigma_schedule(0)
+    L, R, P = operands(core, ctx)
+    S = P.like()
+    packed = lambda: sum(int((x.split() + [1])[2]) for x in launches("{kernel}"))
+    out = []
+    for t, contents in ((None, 1), (None, 2), (L, 2), (None, 2), (None, 3), (R, 3), (None, 3), (None, 4)):
+        if t:
+            t.device_ptr()
+        fake.fake_contents(contents)
+        packed()
+        core.compute_sigma_vector(ctx, L, R, P, S)
+        out.append(packed())
+    """)
+    if precision == "FP64":
+        assert [x - 1 for x in out] == [3, 1, 2, 2, 2, 3, 3, 3]  # (and the packing of L psi)
+    else:
+        assert out == [3, 1, 2, 1, 2, 2, 1, 3]
