@@ -106,6 +106,23 @@ class BlockCache {
     cached_ += bytes;
   }
 
+  // A block whose owner comes back for it under the returned number, unless memory ran short
+  // meanwhile.
+  uint64_t park(void* p, size_t bytes) {
+    std::lock_guard<std::mutex> lk(mu_);
+    parked_[++last_parked_] = {p, bytes};
+    cached_ += bytes;
+    return last_parked_;
+  }
+  bool unpark(uint64_t number) {
+    std::lock_guard<std::mutex> lk(mu_);
+    auto it = parked_.find(number);
+    if (it == parked_.end()) return false;
+    cached_ -= it->second.second;
+    parked_.erase(it);
+    return true;
+  }
+
   void register_stream(cudaStream_t st) {
     std::lock_guard<std::mutex> lk(mu_);
     live_[st] += 1;
@@ -121,15 +138,18 @@ class BlockCache {
     }
   }
 
-  // Free every cached block (cudaFree waits for the device's queued work first).
+  // Free every cached and parked block (cudaFree waits for the device's queued work first).
   void trim() {
     std::multimap<size_t, CachedBlock> blocks;
+    std::map<uint64_t, std::pair<void*, size_t>> parked;
     {
       std::lock_guard<std::mutex> lk(mu_);
       blocks.swap(free_);
+      parked.swap(parked_);
       cached_ = 0;
     }
     for (auto& kv : blocks) cudaFree(kv.second.p);
+    for (auto& kv : parked) cudaFree(kv.second.first);
   }
 
   size_t cached_bytes() {
@@ -141,6 +161,8 @@ class BlockCache {
   std::mutex mu_;
   std::multimap<size_t, CachedBlock> free_;
   std::map<cudaStream_t, int> live_;  // streams of live contexts
+  std::map<uint64_t, std::pair<void*, size_t>> parked_;
+  uint64_t last_parked_ = 0;
   size_t cached_ = 0;
 };
 
@@ -169,6 +191,30 @@ void DevBuf::release() {
   if (p) block_cache().put(p, cap, st);
   p = nullptr;
   cap = 0;
+}
+
+void* Arena::take(size_t bytes, cudaStream_t st) {
+  if (parked_ && !block_cache().unpark(parked_)) p_ = nullptr;
+  parked_ = 0;
+  if (!p_) cap_ = 0;
+  if (p_ && cap_ >= bytes && st_ == st) return p_;
+  if (p_) cudaFree(p_);  // (waits for the work that uses it; not cached: every bond would leave a size)
+  p_ = nullptr;
+  cap_ = 0;
+  p_ = block_cache().get(bytes + bytes / 8, st, &cap_);
+  st_ = st;
+  return p_;
+}
+
+void Arena::park() {
+  if (p_ && !parked_) parked_ = block_cache().park(p_, cap_);
+}
+
+size_t Arena::capacity() const { return cap_; }
+
+Arena::~Arena() {
+  if (parked_ && !block_cache().unpark(parked_)) return;
+  if (p_) block_cache().put(p_, cap_, st_);
 }
 
 namespace {
@@ -1444,12 +1490,11 @@ static void sigma_run_pk_whole(Context& ctx, SigmaPlan& p, double* sigma, PackOp
 }
 
 // FP64 H_eff * psi on the tensor cores: L psi into the FP64 intermediate (stacked panels), the
-// intermediate packed, then the sum over w and B'.  The operators' digits are kept while their
-// data stays.  False: not for these layouts, or no memory for it.
+// intermediate packed, then the sum over w and B'.  The operators' digits serve all products of
+// a call (OzCall).  False: not for these layouts, or no memory for it.
 static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTensor& R, const double* psi,
                          double* sigma) {
   if (!p.stacks) return false;
-  std::vector<std::pair<OzOperand*, const DTensor*>> stale;
   {
     PhaseTimer tm(ctx, kPhSigmaPlan);
     const bool room = oz_reserve(ctx, {&p.o1, &p.o2}, [&] {
@@ -1458,18 +1503,14 @@ static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTe
       return OzScratch{&ctx.scr1, p.o1.tiled_elems * sizeof(double)};
     });
     if (!room) return false;
-    for (auto& x : {std::make_pair(&p.o1.a, &L), std::make_pair(&p.o2.b, &R)}) {
-      if (!x.first->src.is(*x.second, ctx.call)) stale.push_back(x);
-    }
     tm.stop();
     ctx.timers[kPhSigma] -= tm.dt;  // counted as planning, not as H_eff * psi
   }
   double* scr = ctx.scr1.as<double>();
-  std::vector<OzSource> pack;
-  for (const auto& x : stale) pack.push_back(OzSource{x.first, x.second->d});
-  pack.push_back(OzSource{&p.o1.b, psi});
+  std::vector<OzSource> pack{{&p.o1.b, psi}};
+  if (!p.o1.a.cut) pack.push_back({&p.o1.a, L.d});
+  if (!p.o2.b.cut) pack.push_back({&p.o2.b, R.d});
   oz_pack(ctx, pack);
-  for (const auto& x : stale) x.first->src.set(*x.second, ctx.call);  // (queued: they hold these data from here on)
   run_oz_gemm(ctx, p.o1, p.s1, 1.0, L.d, psi, scr, true);
   oz_pack(ctx, {{&p.o2.a, scr}});
   run_oz_gemm(ctx, p.o2, p.s2, 1.0, scr, R.d, sigma, false);
@@ -1662,6 +1703,7 @@ void compute_sigma_vector(Context& ctx, const DTensor& L, const DTensor& R, cons
     throw Error(kInvalidArgument, "compute_sigma_vector: sigma must have the wavefunction's block layout");
   SigmaPlan& p = sigma_plan(ctx, L, R, psi);
   ++ctx.call;
+  OzCall digits(ctx, p.o1, p.o2);
   sigma_run(ctx, p, L, R, psi.d, sigma.d, ctx.precision);
 }
 
@@ -1669,6 +1711,7 @@ double sigma_device_time(Context& ctx, const DTensor& L, const DTensor& R, const
                          int reps) {
   SigmaPlan& p = sigma_plan(ctx, L, R, psi);
   ++ctx.call;
+  OzCall digits(ctx, p.o1, p.o2);
   cudaEvent_t e0, e1;
   cuda_check(cudaEventCreate(&e0), "event create");
   cuda_check(cudaEventCreate(&e1), "event create");
@@ -1798,10 +1841,10 @@ RenormPlan& renorm_plan(Context& ctx, bool forward, const Tensor& opr0, const Te
   return insert_plan(ctx, ctx.renorm_plans, key, build_renorm_plan(ctx, forward, opr0, bra, ket));
 }
 
-// Both FP64 contractions on the tensor cores; every operand is new with each call, its
-// digits go back to the block cache afterwards.  False: no memory for it.
+// Both FP64 contractions on the tensor cores.  False: no memory for it.
 static bool renorm_run_oz(Context& ctx, RenormPlan& rp, const DTensor& bra, const DTensor& opr0, const DTensor& ket,
                           double* scr, double* out) {
+  OzCall digits(ctx, rp.o1, rp.o2);
   const bool room = oz_reserve(ctx, {&rp.o1, &rp.o2}, [&] {
     if (!rp.o1.built) build_oz_gemm(ctx, rp.o1, rp.p1, conj_view(bra), opr0);
     if (!rp.o2.built) build_oz_gemm(ctx, rp.o2, rp.p2, rp.scr, ket);
@@ -1818,8 +1861,6 @@ static bool renorm_run_oz(Context& ctx, RenormPlan& rp, const DTensor& bra, cons
   // no contribution)
   if (rp.p2.c_elems != rp.out.nnz) cuda_check(cudaMemsetAsync(out, 0, rp.out.nnz * sizeof(double), ctx.stream), "renorm zero");
   run_oz_gemm(ctx, rp.o2, rp.p2, 1.0, scr, ket.d, out, true);
-  rp.o1.release();
-  rp.o2.release();
   return true;
 }
 
@@ -2513,6 +2554,7 @@ static double davidson_run(Context& ctx, const DTensor& L, const DTensor& R, con
     throw Error(kInvalidArgument, "diagonalize: diag and wavefunction layouts differ");
   cudaStream_t st = ctx.stream;
   SigmaPlan& sp = sigma_plan(ctx, L, R, wfnc);
+  OzCall digits(ctx, sp.o1, sp.o2);
   ctx.work.ensure(size_t(2 * max_ritz + 1) * std::max<int64_t>(n, 1) * sizeof(double), ctx.stream);
   double* trial = ctx.work.as<double>();
   double* sigma = trial + int64_t(max_ritz) * n;
@@ -2720,8 +2762,6 @@ void release_bond_buffers(Context& ctx) {
       P->buf.release();
       P->src.reset();
     }
-    kv.second->o1.release();
-    kv.second->o2.release();
     kv.second->group_scr.release();
     kv.second->staged.release();
     kv.second->drop_graph();

@@ -43,6 +43,24 @@ struct DevBuf {
   }
 };
 
+// One device buffer that a context's calls use in turn, grown to the largest request.  Between
+// calls it is parked: the memory goes to whoever finds none otherwise.
+class Arena {
+ public:
+  Arena() = default;
+  Arena(const Arena&) = delete;
+  ~Arena();
+  void* take(size_t bytes, cudaStream_t st);
+  void park();
+  size_t capacity() const;  // of the last request
+
+ private:
+  void* p_ = nullptr;
+  size_t cap_ = 0;
+  cudaStream_t st_ = nullptr;
+  uint64_t parked_ = 0;
+};
+
 template <class T>
 struct DevArray {
   DevBuf buf;
@@ -209,7 +227,7 @@ constexpr int kOzTargetTiles = 152 * 8;
 // packing decide.
 constexpr double kOzMinFlops = 1.0e6;
 // packed bytes of a plan that need no look at the free memory (the query is a driver call)
-constexpr int64_t kOzSmallBytes = int64_t(256) << 20;
+constexpr size_t kOzSmallBytes = size_t(256) << 20;
 
 // plans kept per kind in a context before the cache is emptied
 constexpr size_t kMaxCachedPlans = 512;  // default of Context::max_plans
@@ -264,9 +282,11 @@ struct SplitGemm {
   DevArray<DPkPair> pk;
 };
 
-// One operand of a sliced FP64 GEMM: its digit tiles, row exponents and what they hold.
+// One operand of a sliced FP64 GEMM: its digit tiles and row exponents.
 struct OzOperand {
-  DevBuf buf, exps;  // digits; one exponent per packed row
+  uint8_t* digits = nullptr;  // in the context's arena, for the length of a call
+  int* exps = nullptr;        // one exponent per packed row
+  bool cut = false;           // the digits are those of the call's operand
   std::vector<int64_t> base;  // per block slot: byte offset of its tile grid (-1: not packed)
   std::vector<int> exp0, nks;  // per block slot: first exponent, K slices
   std::vector<DOzPack> h_packs;
@@ -277,11 +297,10 @@ struct OzOperand {
   int64_t bytes = 0;
   int rows = 0;
   int seq = 0;  // packings so far
-  PackedSource src;  // what the digits are of
-  void release() {
-    buf.release();
-    exps.release();
-    src.reset();
+  void drop() {
+    digits = nullptr;
+    exps = nullptr;
+    cut = false;
   }
 };
 
@@ -323,9 +342,9 @@ struct OzGemm {
     tiled_elems = 0;
     nslots = 0;
   }
-  void release() {
-    a.release();
-    b.release();
+  void drop() {
+    a.drop();
+    b.drop();
   }
 };
 // tiled_out: the result goes to a tiled intermediate (stacked, unswapped plans); from: the
@@ -343,12 +362,23 @@ void run_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, double alpha, cons
                  bool assign);
 // Device memory of a product's plans, which `build` makes where they are not built: their
 // packed operands, split-K slots and the scratch that it returns.  False where that would
-// take more than half of what is free, or where an allocation fails (nothing is held then).
+// leave less than an eighth of what is free, or where an allocation fails.
 struct OzScratch {
   DevBuf* buf = nullptr;
   size_t bytes = 0;
 };
 bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs, const std::function<OzScratch()>& build);
+// The digits of a call's products: they end with it.
+class OzCall {
+ public:
+  OzCall(Context& ctx, OzGemm& a, OzGemm& b) : ctx_(ctx), a_(a), b_(b) {}
+  OzCall(const OzCall&) = delete;
+  ~OzCall();
+
+ private:
+  Context& ctx_;
+  OzGemm &a_, &b_;
+};
 // whether a plan of that many FLOPs runs on the tensor cores
 bool oz_wanted(const Context& ctx, double flops);
 // Output tiles of every task with long pair lists split along K (engine.cpp)
@@ -518,6 +548,7 @@ struct Context {
   DevBuf partial;    // reduction partials
   DevBuf scalars;    // small device scalars
   DevBuf dv_sums;    // Davidson: ticket, sums and partials of the fused vector kernels
+  Arena oz_mem;      // digits of the sliced FP64 products
   DevBuf print_sums; // fingerprints: sums and counts of CTAs
   cudaEvent_t dv_done = nullptr;
   DevBuf svd_work;   // solver workspace

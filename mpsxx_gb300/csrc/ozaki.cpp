@@ -251,32 +251,47 @@ bool oz_wanted(const Context& ctx, double flops) {
 bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs, const std::function<OzScratch()>& build) {
   try {
     const OzScratch scratch = build();
-    std::vector<std::pair<DevBuf*, size_t>> bufs;
-    size_t part = 16;
+    bool held = true;
+    size_t digits = 0, part = 16;
+    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
     for (OzGemm* g : gs) {
       for (OzOperand* o : {&g->a, &g->b}) {
-        bufs.push_back({&o->buf, std::max<int64_t>(o->bytes, 16)});
-        bufs.push_back({&o->exps, size_t(std::max(o->rows, 1)) * sizeof(int)});
+        held = held && o->digits != nullptr;
+        digits += up(o->bytes + 16) + up(o->rows * sizeof(int) + 16);
       }
       part = std::max(part, g->partial_bytes());
     }
-    bufs.push_back({&ctx.gemm_part, part});
-    if (scratch.buf) bufs.push_back({scratch.buf, std::max<size_t>(scratch.bytes, 16)});
-    int64_t need = 0;
-    for (const auto& b : bufs)
-      if (b.first->cap < b.second) need += static_cast<int64_t>(b.second);
+    size_t need = (held ? 0 : digits) + (ctx.gemm_part.cap < part ? part : 0);
+    if (scratch.buf && scratch.buf->cap < scratch.bytes) need += scratch.bytes;
     if (need > kOzSmallBytes) {
       size_t free_b = 0, total_b = 0;
       cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-      if (need > static_cast<int64_t>((free_b + block_cache_bytes()) / 2)) return false;
+      const size_t have = free_b + block_cache_bytes();
+      if (need > have - have / 8) return false;
     }
-    for (const auto& b : bufs) b.first->ensure(b.second, ctx.stream);
+    ctx.gemm_part.ensure(part, ctx.stream);
+    if (scratch.buf) scratch.buf->ensure(std::max<size_t>(scratch.bytes, 16), ctx.stream);
+    if (held) return true;
+    uint8_t* at = static_cast<uint8_t*>(ctx.oz_mem.take(digits, ctx.stream));
+    for (OzGemm* g : gs)
+      for (OzOperand* o : {&g->a, &g->b}) {
+        o->drop();
+        o->digits = at;
+        at += up(o->bytes + 16);
+        o->exps = reinterpret_cast<int*>(at);
+        at += up(o->rows * sizeof(int) + 16);
+      }
   } catch (const Error& e) {
     if (e.code != kAlloc) throw;
-    for (OzGemm* g : gs) g->release();
     return false;
   }
   return true;
+}
+
+OzCall::~OzCall() {
+  a_.drop();
+  b_.drop();
+  ctx_.oz_mem.park();
 }
 
 void oz_pack(Context& ctx, const std::vector<OzSource>& what) {
@@ -284,21 +299,23 @@ void oz_pack(Context& ctx, const std::vector<OzSource>& what) {
   OzPackJobs jobs{};
   for (const OzSource& w : what) {
     OzOperand& o = *w.o;
-    jobs.job[jobs.n++] = OzPackJob{o.packs.get(), o.segs.get(), w.src, o.buf.as<uint8_t>(), o.exps.as<int>(),
-                                   o.flag.get(), static_cast<int>(o.h_packs.size()), o.seq + 1};
+    jobs.job[jobs.n++] = OzPackJob{o.packs.get(), o.segs.get(), w.src, o.digits, o.exps, o.flag.get(), static_cast<int>(o.h_packs.size()), o.seq + 1};
   }
   launch_oz_pack(jobs, ctx.stream);
-  for (const OzSource& w : what) ++w.o->seq;
+  for (const OzSource& w : what) {
+    ++w.o->seq;
+    w.o->cut = true;
+  }
   ctx.kernel_launches += 1;
 }
 
 void run_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, double alpha, const double* A, const double* B, double* C,
                  bool assign) {
   OzGemmArgs a{};
-  a.Apk = og.a.buf.as<uint8_t>();
-  a.Bpk = og.b.buf.as<uint8_t>();
-  a.Aexp = og.a.exps.as<int>();
-  a.Bexp = og.b.exps.as<int>();
+  a.Apk = og.a.digits;
+  a.Bpk = og.b.digits;
+  a.Aexp = og.a.exps;
+  a.Bexp = og.b.exps;
   a.flag_a = og.a.flag.get();
   a.flag_b = og.b.flag.get();
   a.seq_a = og.a.seq;

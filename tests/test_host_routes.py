@@ -80,7 +80,7 @@ def test_a_launch_that_fails_while_a_graph_is_captured():
 
 def test_products_after_an_allocation_that_failed():
     """Whichever allocation of a sliced product fails, the call gives a result on the FP64 pipe or
-    an allocation error, and the next one cuts the digits that the first did not."""
+    an allocation error, and the next one cuts all digits."""
     out = run("""
     out = []
     for k in range(40):
@@ -107,15 +107,14 @@ def test_products_after_an_allocation_that_failed():
         assert code in (0, 2) and code2 == 0
         if code == 0:
             assert (pipe, first) in ((2, []), (0, [3, 1]))
-        # L, R and psi; psi alone where L's and R's digits are there
-        assert second == ([1, 1] if 3 in first else [3, 1])
+        assert second == [3, 1]  # L, R and psi, then L psi
 
 
 @pytest.mark.parametrize("precision, kernel", [("FP64", "oz_pack_kernel"), ("SPLIT_TF32", "pack_kernelEPKNS_5DPack")])
 def test_operators_are_packed_anew_where_a_caller_may_have_written_them(precision, kernel):
-    """Packed operators are kept between products.  Of a tensor whose device pointer was handed
-    out the data may be other data in every call: digits are cut anew, split operators packed
-    anew where their fingerprint is another one (or none was taken of the packed data)."""
+    """Digits are cut in every call.  Packed split operators are kept; of a tensor whose device
+    pointer was handed out the data may be other data in every call: it is packed anew where
+    its fingerprint is another one (or none was taken of the packed data)."""
     out = run(f"""
     ctx = core.Context(0)
     core.set_precision(ctx, core.{precision})
@@ -134,6 +133,41 @@ def test_operators_are_packed_anew_where_a_caller_may_have_written_them(precisio
         out.append(packed())
     """)
     if precision == "FP64":
-        assert [x - 1 for x in out] == [3, 1, 2, 2, 2, 3, 3, 3]  # (and the packing of L psi)
+        assert [x - 1 for x in out] == 8 * [3]  # (and the packing of L psi)
     else:
         assert out == [3, 1, 2, 1, 2, 2, 1, 3]
+
+
+def test_memory_of_the_digits():
+    """One bond's digits at most are held, and only until memory is short; a product without
+    memory for them runs on the FP64 pipe."""
+    out = run("""
+    ctx = core.Context(0)
+    ctx.set_fp64_route(0.0)
+    empty_cache(ctx)
+    bonds = [operands(core, ctx, (400 - 30 * k, 60 * k + 20)) for k in range(5)]
+    small = operands(core, ctx, (9, 30))
+    def product(b):
+        launches()
+        code = error(core.compute_sigma_vector, ctx, *b, b[2].like())
+        ran = launches()
+        return [code] + [sum(k in x for x in ran) for k in ("gemm_oz", "gemm_f64")]
+    bonds.sort(key=lambda b: -b[0].nnz - b[1].nnz)
+    product(small)
+    used = [fake.fake_used()]
+    runs = [product(bonds[0])]
+    used.append(fake.fake_used())
+    runs += [product(b) for b in bonds + bonds[::-1]]
+    used.append(fake.fake_used())
+    # a tensor for which there is room only where the digits were
+    fake.fake_limit(fake.fake_used())
+    n = 7 * (bonds[0][0].nnz + bonds[0][1].nnz)  # half of L's and R's digits
+    t = core.Tensor.create(ctx, (0, 0), [[(0, 0)]], [[n // 8]])
+    short = product(bonds[0])
+    fake.fake_limit(0)
+    out = [runs, used, short, product(bonds[0])]
+    """)
+    runs, used, short, after = out
+    assert runs == 11 * [[0, 2, 0]]
+    assert used[2] - used[1] < (used[1] - used[0]) // 4  # the other nine products add no digits
+    assert short == [0, 0, 2] and after == [0, 2, 0]
