@@ -193,7 +193,7 @@ void launch_fingerprints(const PrintJobs& jobs, int njobs, unsigned long long* s
 // slice of 16 the seven digits' rows x 16 bf16.  Padding rows are not written.
 constexpr int kOzTileM = 128, kOzTileN = 32, kOzTileK = 16, kOzDigits = 7;
 constexpr int kOzGroupSteps = 10;     // K slices summed in one FP32 accumulation (exact up to 160)
-constexpr int kOzMaxExponent = 480;   // rows of larger magnitude flag their operand
+constexpr int kOzMaxExponent = 480;   // rows of magnitudes outside 2^-480 .. 2^480 flag their operand
 constexpr uint32_t kOzTileABytes = kOzDigits * kOzTileM * kOzTileK * 2;
 constexpr uint32_t kOzTileBBytes = kOzDigits * kOzTileN * kOzTileK * 2;
 __host__ __device__ constexpr int oz_tile_rows(int rows, int tm) {

@@ -32,10 +32,10 @@
 // ring; warp 1 lane 0 issues the MMAs; warps 4-19 are the epilogue (warp 4 + 4 c + q:
 // tensor-memory lanes 32 q.., output columns 8 c..).
 //
-// A row with a value that is not finite or of 2^480 and above sets the operand's flag; the
-// kernel then computes its tiles from the FP64 operands directly (plain loops: such operands
-// do not occur in a converging sweep, but give what FP64 arithmetic gives).  Rows below
-// 2^-480 keep that scale.
+// A row with a value that is not finite or of 2^480 and above, or of values below 2^-480 that
+// are not all zero, sets the operand's flag; the kernel then computes its tiles from the FP64
+// operands directly (plain loops: such operands do not occur in a converging sweep, but give
+// what FP64 arithmetic gives).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -551,9 +551,13 @@ __global__ void __launch_bounds__(256, 4) oz_pack_kernel(const OzPackJobs jobs) 
     for (int i = 0; i < 8; ++i) x[i] = i < n ? p[(long long)i * ks] : 0.0;
   };
   auto top = [&](const double (&x)[8], int r) {
-    int m = 0;
+    int m = 0, low = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) m = max(m, __double2hiint(x[i]) & 0x7fffffff);
+    for (int i = 0; i < 8; ++i) {
+      m = max(m, __double2hiint(x[i]) & 0x7fffffff);
+      low |= __double2loint(x[i]);
+    }
+    if (m == 0 && low != 0) m = 1;  // (the smallest subnormal numbers)
     if (m) atomicMax(&row_max[r], m);
   };
   auto emit = [&](const double (&x)[8], int r, int kg) {
@@ -606,9 +610,11 @@ __global__ void __launch_bounds__(256, 4) oz_pack_kernel(const OzPackJobs jobs) 
   }
   __syncthreads();
   if (threadIdx.x < pk.rows) {
-    const int e = row_exponent(row_max[threadIdx.x] >> 20);
+    const int m = row_max[threadIdx.x], e = row_exponent(m >> 20);
     job.exps[pk.exp0 + threadIdx.x] = e;
-    if (e > kOzMaxExponent) atomicMax(job.flag, job.seq);  // (a value that is not finite has the largest exponent)
+    // out of range: the largest magnitude 2^480 or above (also of a value that is not finite),
+    // or below 2^-480 and not zero
+    if (e > kOzMaxExponent || (m != 0 && (m >> 20) - 1022 < -kOzMaxExponent)) atomicMax(job.flag, job.seq);
   }
 #pragma unroll
   for (int h = 0; h < kHold; ++h)

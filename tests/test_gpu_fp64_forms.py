@@ -16,6 +16,7 @@ pytestmark = pytest.mark.gpu
 FORMS = {
     "repeated": ([70, 3, 130, 41], [33, 64, 17, 20], [(0, 0), (0, 0), (1, 0), (0, 0)]),
     "repeated-columns": ([5, 9, 16], [40, 2, 7], [(1, 0), (0, 0), (1, 0)]),
+    "plain": ([5, 9, 16], [40, 2, 7], [(0, 0), (1, 0), (2, 0)]),
     "empty": ([70, 0, 41], [33, 17, 0], [(0, 0), (1, 0), (2, 0)]),
     "one": ([1, 1], [1, 1], [(0, 0), (0, 0)]),
 }
@@ -94,3 +95,32 @@ def test_products(ctx, form, route):
         du = core.Tensor.from_dict(ctx, to_dict(u))
         got = core.renormalize(ctx, forward, d[opr], du, du)
         check(got.to_blocks(), od.renormalize_merged(forward, strip[opr], u, u))
+
+
+@pytest.mark.parametrize("small, big", [(-470, 400), (-500, 400), (-560, 460), (-1000, 470), (-1060, 470)])
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_rows_of_small_numbers(ctx, which, small, big):
+    """Rows below the range of the digits (2^-480), down to subnormal numbers, are computed like any
+    others: the FP64 pipe's result up to the rounding of sums of at most 16 and 3 x 40 terms, whose
+    magnitudes are at most 16 times the largest result's."""
+    from mpsxx_gb300 import core
+
+    x = bond("plain", seed=3)
+    rng = np.random.default_rng(which)
+    for i, a in enumerate(x):
+        e = {which: small, (which + 1) % 3: big}.get(i, 0)
+        for t, b in a.blocks.items():
+            row = np.ones(b.shape[0])
+            if i == which:
+                row[rng.random(b.shape[0]) < 0.3] = 0.0  # rows of zeros among them
+            a.blocks[t] = np.ldexp(b, e) * row.reshape([-1] + [1] * (b.ndim - 1))
+    res = []
+    for route in (float("inf"), 0.0):
+        ctx.set_fp64_route(route)
+        d = [core.Tensor.from_dict(ctx, to_dict(a)) for a in x]
+        S = d[2].like()
+        core.compute_sigma_vector(ctx, *d, S)
+        res.append(S.download())
+    top = np.abs(res[0]).max()
+    assert top > 0.0
+    assert np.max(np.abs(res[1] - res[0])) <= 1e-13 * top
