@@ -128,8 +128,16 @@ int mpsxx_context_set_sigma_operator_format(mpsxx_context* ctx, int fp32_operato
  * off. */
 int mpsxx_context_set_svd_routes(mpsxx_context* ctx, int jacobi_max_cols, int gram_max_dim);
 /* FP64 H_eff*psi and renormalisations of at least min_flops floating-point operations run
- * on the tensor cores (error-free slicing, FP64 accuracy), smaller ones on the FP64 pipe;
- * negative: the default; 0: all on the tensor cores; infinity: none. */
+ * on the tensor cores (operands sliced into digits), smaller ones on the FP64 pipe;
+ * negative: the default; 0: all on the tensor cores; infinity: none.
+ * A sliced sum of K products is off by at most K 2^-53 of (largest magnitude of the row x
+ * largest magnitude of the column); FP64 multiply-adds are by K 2^-53 of the sum of
+ * magnitudes.  So that the two are close, the contractions of compute_sigma_vector and of
+ * renormalisations are balanced by powers of two first (the largest magnitudes of the
+ * wavefunction's rows and columns, of the site tensors' contracted index); diagonalize, whose
+ * vectors enter through norms and dot products, slices its operators once, unbalanced.
+ * Where an element that is small against both maxima needs a small error of its own, the
+ * FP64 pipe gives it. */
 int mpsxx_context_set_fp64_route(mpsxx_context* ctx, double min_flops);
 /* Plans (H_eff*psi, diagonal, merged-operator, renormalisation) kept per kind before
  * the context empties a cache (default 512).  Plans are keyed by structural layouts,

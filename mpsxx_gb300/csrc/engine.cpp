@@ -1493,13 +1493,14 @@ static void sigma_run_pk_whole(Context& ctx, SigmaPlan& p, double* sigma, PackOp
 // intermediate packed, then the sum over w and B'.  The operators' digits serve all products of
 // a call (OzCall).  False: not for these layouts, or no memory for it.
 static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTensor& R, const double* psi,
-                         double* sigma) {
+                         double* sigma, bool balanced) {
   if (!p.stacks) return false;
   {
     PhaseTimer tm(ctx, kPhSigmaPlan);
     const bool room = oz_reserve(ctx, {&p.o1, &p.o2}, [&] {
-      if (!p.o1.built) build_oz_gemm(ctx, p.o1, p.s1, L, p.psi_layout, true);
-      if (!p.o2.built) build_oz_gemm(ctx, p.o2, p.s2, p.scr1, R, false, &p.o1, &p.s1);
+      const Tensor& w = p.psi_layout;
+      if (!p.o1.built) build_oz_gemm(ctx, p.o1, p.s1, L, w, OzBalance{w, 0, 2, 0, 1}, true);
+      if (!p.o2.built) build_oz_gemm(ctx, p.o2, p.s2, p.scr1, R, OzBalance{w, 1, 2, 2, -1, 1, 1}, false, &p.o1, &p.s1);
       return OzScratch{&ctx.scr1, p.o1.tiled_elems * sizeof(double)};
     });
     if (!room) return false;
@@ -1507,21 +1508,24 @@ static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTe
     ctx.timers[kPhSigma] -= tm.dt;  // counted as planning, not as H_eff * psi
   }
   double* scr = ctx.scr1.as<double>();
-  std::vector<OzSource> pack{{&p.o1.b, psi}};
-  if (!p.o1.a.cut) pack.push_back({&p.o1.a, L.d});
-  if (!p.o2.b.cut) pack.push_back({&p.o2.b, R.d});
+  const OzGemm *bal1 = balanced ? &p.o1 : nullptr, *bal2 = balanced ? &p.o2 : nullptr;
+  if (balanced) oz_scale(ctx, {{&p.o1, psi}, {&p.o2, psi}});
+  std::vector<OzSource> pack{{&p.o1.b, psi, bal1}};
+  if (!p.o1.a.cut) pack.push_back({&p.o1.a, L.d, bal1});
+  if (!p.o2.b.cut) pack.push_back({&p.o2.b, R.d, bal2});
   oz_pack(ctx, pack);
   run_oz_gemm(ctx, p.o1, p.s1, 1.0, L.d, psi, scr, true);
-  oz_pack(ctx, {{&p.o2.a, scr}});
+  oz_pack(ctx, {{&p.o2.a, scr, bal2}});
   run_oz_gemm(ctx, p.o2, p.s2, 1.0, scr, R.d, sigma, false);
   return true;
 }
 
+// balanced: the one product of its call, whose FP64 contractions are balanced
 static void sigma_run(Context& ctx, SigmaPlan& p, const DTensor& L, const DTensor& R, const double* psi,
-                      double* sigma, int precision) {
+                      double* sigma, int precision, bool balanced = false) {
   if (precision != kFP64) {
     sigma_run_pk(ctx, p, L, R, psi, sigma);
-  } else if (oz_wanted(ctx, p.flops) && sigma_run_oz(ctx, p, L, R, psi, sigma)) {
+  } else if (oz_wanted(ctx, p.flops) && sigma_run_oz(ctx, p, L, R, psi, sigma, balanced)) {
   } else {
     ctx.scr1.ensure(std::max<int64_t>(p.scr1.nnz, 1) * sizeof(double), ctx.stream);
     double* scr = ctx.scr1.as<double>();
@@ -1704,7 +1708,7 @@ void compute_sigma_vector(Context& ctx, const DTensor& L, const DTensor& R, cons
   SigmaPlan& p = sigma_plan(ctx, L, R, psi);
   ++ctx.call;
   OzCall digits(ctx, p.o1, p.o2);
-  sigma_run(ctx, p, L, R, psi.d, sigma.d, ctx.precision);
+  sigma_run(ctx, p, L, R, psi.d, sigma.d, ctx.precision, true);
 }
 
 double sigma_device_time(Context& ctx, const DTensor& L, const DTensor& R, const DTensor& psi, DTensor& sigma,
@@ -1846,17 +1850,19 @@ static bool renorm_run_oz(Context& ctx, RenormPlan& rp, const DTensor& bra, cons
                           double* scr, double* out) {
   OzCall digits(ctx, rp.o1, rp.o2);
   const bool room = oz_reserve(ctx, {&rp.o1, &rp.o2}, [&] {
-    if (!rp.o1.built) build_oz_gemm(ctx, rp.o1, rp.p1, conj_view(bra), opr0);
-    if (!rp.o2.built) build_oz_gemm(ctx, rp.o2, rp.p2, rp.scr, ket);
+    const int ax = rp.p1.ta == kTrans ? 0 : 1;  // the index of bra and ket that is contracted
+    if (!rp.o1.built) build_oz_gemm(ctx, rp.o1, rp.p1, conj_view(bra), opr0, OzBalance{bra, ax, ax, 0, -1});
+    if (!rp.o2.built) build_oz_gemm(ctx, rp.o2, rp.p2, rp.scr, ket, OzBalance{ket, ax, 2, ax, 1});
     return OzScratch{};
   });
   if (!room) return false;
-  oz_pack(ctx, {{&rp.o1.a, rp.o1.swap ? opr0.d : bra.d},
-                {&rp.o1.b, rp.o1.swap ? bra.d : opr0.d},
-                {rp.o2.swap ? &rp.o2.a : &rp.o2.b, ket.d}});
+  oz_scale(ctx, {{&rp.o1, bra.d}, {&rp.o2, ket.d}});
+  oz_pack(ctx, {{&rp.o1.a, rp.o1.swap ? opr0.d : bra.d, &rp.o1},
+                {&rp.o1.b, rp.o1.swap ? bra.d : opr0.d, &rp.o1},
+                {rp.o2.swap ? &rp.o2.a : &rp.o2.b, ket.d, &rp.o2}});
   if (!rp.p1.full) cuda_check(cudaMemsetAsync(scr, 0, rp.scr.nnz * sizeof(double), ctx.stream), "renorm scr zero");
   run_oz_gemm(ctx, rp.o1, rp.p1, 1.0, bra.d, opr0.d, scr, true);
-  oz_pack(ctx, {{rp.o2.swap ? &rp.o2.b : &rp.o2.a, scr}});
+  oz_pack(ctx, {{rp.o2.swap ? &rp.o2.b : &rp.o2.a, scr, &rp.o2}});
   // (the result is new: its blocks are written, not added to, and zeroed only where some have
   // no contribution)
   if (rp.p2.c_elems != rp.out.nnz) cuda_check(cudaMemsetAsync(out, 0, rp.out.nnz * sizeof(double), ctx.stream), "renorm zero");

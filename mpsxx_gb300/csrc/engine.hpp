@@ -296,7 +296,8 @@ struct OzOperand {
   DevView<int> flag;  // number of the last packing that met a value which cannot be sliced
   int64_t bytes = 0;
   int rows = 0;
-  int seq = 0;  // packings so far
+  int seq = 0;   // packings so far
+  int sign = 0;  // of the powers of two
   void drop() {
     digits = nullptr;
     exps = nullptr;
@@ -328,6 +329,11 @@ struct OzGemm {
   std::vector<DOzTiled> task_place;
   int64_t tiled_elems = 0;
   DevView<DOzTiled> pairs_tiled;
+  // powers of two that balance the contraction (OzBalance), made with each product that uses them
+  std::vector<DOzScale> h_scale_tasks;
+  DevView<DOzScale> scale_tasks;
+  DevView<DOzScaleBlock> scale_blocks;
+  DevView<int8_t> scales;
   size_t partial_bytes() const { return size_t(nslots) * kOzTileM * kOzTileN * sizeof(double); }
   void clear() {  // what a build that did not end has left
     for (OzOperand* o : {&a, &b}) {
@@ -336,6 +342,7 @@ struct OzGemm {
       o->bytes = 0;
       o->rows = 0;
     }
+    h_scale_tasks.clear();
     h_tiles.clear();
     h_reduce.clear();
     task_place.clear();
@@ -347,16 +354,28 @@ struct OzGemm {
     b.drop();
   }
 };
+// What balances a contraction (kernels_oz.cu): the largest magnitudes of `of`, a two-index
+// array, along `axis`; the contraction is over that index as axis_a of A's and axis_b of B's,
+// after the index w_a of A's and w_b of B's where there are two (-1: one).  A's elements are
+// multiplied by 2^(sign_a e), B's by 2^(-sign_a e).
+struct OzBalance {
+  const Tensor& of;
+  int axis, axis_a, axis_b, sign_a;
+  int w_a = -1, w_b = -1;
+};
 // tiled_out: the result goes to a tiled intermediate (stacked, unswapped plans); from: the
 // plan whose tiled result is this one's A (blocks of `a` matched by from's task result tags).
-void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a, const Tensor& b, bool tiled_out = false,
-                   const OzGemm* from = nullptr, const GemmPlan* from_plan = nullptr);
+void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a, const Tensor& b, const OzBalance& bal,
+                   bool tiled_out = false, const OzGemm* from = nullptr, const GemmPlan* from_plan = nullptr);
 // Packs operands of built plans from FP64 data, up to kOzPackJobs in one launch.
 struct OzSource {
   OzOperand* o;
   const double* src;
+  const OzGemm* balance = nullptr;  // the plan whose powers of two apply (all of a launch's operands or none)
 };
 void oz_pack(Context& ctx, const std::vector<OzSource>& what);
+// The powers of two of up to two plans from the arrays that their OzBalance names.
+void oz_scale(Context& ctx, const std::vector<std::pair<OzGemm*, const double*>>& what);
 // C = (assign) or += alpha op(A) op(B) from the packed operands.
 void run_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, double alpha, const double* A, const double* B, double* C,
                  bool assign);

@@ -204,10 +204,11 @@ __host__ __device__ constexpr int oz_tail_cols(int rows, int tn) {
 }
 // A CTA's rows [row0, row0 + rows) of an operand block (or panel), a multiple of 8: the
 // block's tiles of 1 << tile_log2 rows (the last, tile `last`, of tail rows) start at dst_off;
-// the rows' exponents go to exps[exp0..].
+// the rows' exponents go to exps[exp0..].  scale: the first of the contraction's powers of two
+// (launch_oz_scale).
 struct DOzPack {
   int64_t dst_off;
-  int seg0, nseg, rows, row0, k, nks, exp0, tile_log2, last, tail;
+  int seg0, nseg, rows, row0, k, nks, exp0, tile_log2, last, tail, scale;
 };
 constexpr int kOzPackRows = 128, kOzPackElems = 4096;
 // CTA rows [row, row + n): element (i, k) at src_off + i rstride + k kstride; kstride 0: the
@@ -266,6 +267,9 @@ struct OzPackJob {
   uint8_t* dst;
   int *exps, *flag;
   int npacks, seq;
+  // unless null, the element at k of the contraction counts 2^(sign scales[k]) times
+  const int8_t* scales;
+  int sign;
 };
 constexpr int kOzPackJobs = 3;
 struct OzPackJobs {
@@ -273,6 +277,28 @@ struct OzPackJobs {
   int n;
 };
 void launch_oz_pack(const OzPackJobs& jobs, cudaStream_t st);
+// A contraction's powers of two, 32 entries from i0 of its dim: the exponent of the largest
+// magnitude among the elements off + i istride + l lstride, l < len, of blocks [b0, b1), at most
+// 127 either way, -127 for zeros; written repeat times, dim entries apart, from out on.
+struct DOzScaleBlock {
+  int64_t off;
+  int len, istride, lstride;
+};
+struct DOzScale {
+  int out, dim, repeat, i0, b0, b1;
+};
+struct OzScaleJob {
+  const DOzScale* tasks;
+  const DOzScaleBlock* blocks;
+  const double* src;
+  int8_t* out;
+  int ntasks;
+};
+struct OzScaleJobs {
+  OzScaleJob job[2];
+  int n;
+};
+void launch_oz_scale(const OzScaleJobs& jobs, cudaStream_t st);
 
 void launch_gemm_f64(int transa, int transb, double alpha, const double* A, const double* B, double* C,
                      const DTile* tiles, int ntiles, const DGemmTask* tasks, const DGemmPair* pairs,

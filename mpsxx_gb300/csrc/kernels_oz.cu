@@ -9,11 +9,24 @@
 // exactly by the FP32 accumulators, all products of one weight (p + q = t + 2, t = 0..7)
 // in one accumulator: at most 7 x 160 products of 2^14 for a contraction of 160, below
 // 2^24 but for the last weights, where a rounding is under the dropped products.  The 34
-// products with p + q <= 9 are kept; what is dropped or rounded is below 2^-61 of (row
-// maximum x column maximum) per product, and the sums carry no rounding.  Measured
-// against 80-bit sums on blocks of 1..234 terms, Gaussian or decaying over four decades
-// along rows, columns or the contraction: 5e-17 .. 1.2e-16 relative, a chain of FP64
-// fused multiply-adds 4e-17 .. 6e-16.
+// products with p + q <= 9 are kept.  An operand is off by at most half a unit of 2^(e-55) (e
+// the exponent of its row), the sum of a group of 160 by half a unit of 2^(e-55) (e the sum of
+// both exponents), what is dropped is below 2^-61 of 2^e: a sum of K products by at most
+// K 2^-53 of (row maximum x column maximum).  FP64 multiply-adds are off by at most K 2^-53 of
+// the sum of magnitudes, which is less where large elements of a row meet small ones of a
+// column.
+//
+// Contractions are balanced for that reason: the elements at k are multiplied by 2^s_k in
+// one operand and 2^-s_k in the other while they are sliced, s_k the exponent of the largest
+// magnitude at k of the wavefunction (for both of its indices) or of a site tensor
+// (oz_scale_kernel).  Largest error of an element of H_eff*psi relative to its sum of magnitudes,
+// without / with / FP64 pipe: on converged Hubbard bonds (M=32, 64) 5e-13 .. 6e-10 / 1.4e-15 ..
+// 1e-13 / 2.5e-16; on wavefunctions graded over four decades, Hubbard M=33..101 5e-15 .. 1e-14 /
+// 3e-16 .. 7e-16 / 3e-16 .. 5e-16, QC M=40, 60 2e-16 / 2e-16 / 5e-16; rms values below the FP64
+// pipe's but for the converged bonds (1e-16 .. 6e-15 / 5e-17).  It costs the launch of the maxima
+// and 6 of some 50 instructions an element of the packing: 55 -> 57 us at Hubbard M=64, 136 -> 143
+// at M=512, 7.68 -> 7.92 ms at QC n=20 M=512.  An eigenproblem, whose operators are sliced once and
+// whose vectors enter through norms and dot products, does not balance.
 //
 // A K step of 16 is seven MMAs: digit p of A times the stacked digits [B_1; ..; B_n] as
 // one operand, written at the accumulator columns of weight p - 1, so that every product
@@ -24,8 +37,8 @@
 // next group of K steps issues.
 //
 // H_eff*psi at the C2 size (QC n=20 M=512, 88 GFLOP): 91.5 ms on the FP64 pipe (0.96 TFLOP/s,
-// 89 % of cuBLAS DGEMM), 7.7 ms sliced with both operators packed anew (11 TFLOP/s; GEMMs 5.5
-// ms, packing 2.2), 137 us against 1.25 ms at Hubbard M=512.
+// 89 % of cuBLAS DGEMM), 7.9 ms sliced (11 TFLOP/s; GEMMs 5.5 ms, packing 2.4), 143 us against
+// 1.25 ms at Hubbard M=512.
 //
 // GEMM CTA (640 threads, warp-specialised, persistent over the tile list): warp 0 lane 0
 // copies operand slices (one bulk copy each of A and B per K step) into a six-stage
@@ -496,7 +509,9 @@ __device__ __forceinline__ unsigned long long biased56(double x, int e1022) {
 // 2199 us for a renormalisation at QC n=20 M=512 and 7.88 -> 7.68 ms for its H_eff*psi; five with one
 // item held lose it again to the second reads (2394 us, 7.97 ms).
 constexpr int kHold = 2;
-__global__ void __launch_bounds__(256, 4) oz_pack_kernel(const OzPackJobs jobs) {
+template <bool kScaled>
+__global__ void __launch_bounds__(256, 4) oz_pack_kernel(const __grid_constant__ OzPackJobs jobs) {
+  constexpr int kExp = kScaled ? 16 : 20;  // row_max holds an exponent from this bit on
   __shared__ long long row_off[kOzPackRows];
   __shared__ int row_ks[kOzPackRows];
   __shared__ int row_max[kOzPackRows];
@@ -550,22 +565,36 @@ __global__ void __launch_bounds__(256, 4) oz_pack_kernel(const OzPackJobs jobs) 
 #pragma unroll
     for (int i = 0; i < 8; ++i) x[i] = i < n ? p[(long long)i * ks] : 0.0;
   };
-  auto top = [&](const double (&x)[8], int r) {
+  // the 8 powers of two of a K group as bytes
+  auto powers = [&](int kg) {
+    uint2 p = make_uint2(0, 0);
+    if (kScaled) {
+      p = *reinterpret_cast<const uint2*>(job.scales + pk.scale + kg * 8);
+      if (job.sign < 0) p = make_uint2(__vneg4(p.x), __vneg4(p.y));
+    }
+    return p;
+  };
+  auto power = [](const uint2& p, int i) { return (int)(int8_t)((i < 4 ? p.x : p.y) >> (8 * (i & 3))); };
+  auto top = [&](const double (&x)[8], int r, int kg) {
     int m = 0, low = 0;
+    const uint2 p = powers(kg);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      m = max(m, __double2hiint(x[i]) & 0x7fffffff);
+      int h = __double2hiint(x[i]) & 0x7fffffff;
+      if (kScaled && h != 0) h = max((h >> 4) + power(p, i) * (1 << kExp), 1);  // (>> 4: room for the largest)
+      m = max(m, h);
       low |= __double2loint(x[i]);
     }
     if (m == 0 && low != 0) m = 1;  // (the smallest subnormal numbers)
     if (m) atomicMax(&row_max[r], m);
   };
   auto emit = [&](const double (&x)[8], int r, int kg) {
-    const int e1022 = row_exponent(row_max[r] >> 20) + 1022;
+    const int e1022 = row_exponent(row_max[r] >> kExp) + 1022;
+    const uint2 pw = powers(kg);
     uint32_t lo[8], hi[8];  // bytes: digit + 128 (the leading one in the upper 16 bits)
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const unsigned long long d = biased56(x[i], e1022);
+      const unsigned long long d = biased56(x[i], kScaled ? e1022 - power(pw, i) : e1022);
       lo[i] = (uint32_t)d;
       hi[i] = (uint32_t)(d >> 32);
     }
@@ -600,21 +629,21 @@ __global__ void __launch_bounds__(256, 4) oz_pack_kernel(const OzPackJobs jobs) 
   }
 #pragma unroll
   for (int h = 0; h < kHold; ++h)
-    if (threadIdx.x + h * 256 < items) top(x[h], rr[h]);
+    if (threadIdx.x + h * 256 < items) top(x[h], rr[h], kk[h]);
   for (int it = threadIdx.x + kHold * 256; it < items; it += 256) {
     double y[8];
     int r, kg;
     place(it, r, kg);
     fetch(r, kg, y);
-    top(y, r);
+    top(y, r, kg);
   }
   __syncthreads();
   if (threadIdx.x < pk.rows) {
-    const int m = row_max[threadIdx.x], e = row_exponent(m >> 20);
+    const int m = row_max[threadIdx.x], e = row_exponent(m >> kExp);
     job.exps[pk.exp0 + threadIdx.x] = e;
     // out of range: the largest magnitude 2^480 or above (also of a value that is not finite),
     // or below 2^-480 and not zero
-    if (e > kOzMaxExponent || (m != 0 && (m >> 20) - 1022 < -kOzMaxExponent)) atomicMax(job.flag, job.seq);
+    if (e > kOzMaxExponent || (m != 0 && (m >> kExp) - 1022 < -kOzMaxExponent)) atomicMax(job.flag, job.seq);
   }
 #pragma unroll
   for (int h = 0; h < kHold; ++h)
@@ -628,7 +657,48 @@ __global__ void __launch_bounds__(256, 4) oz_pack_kernel(const OzPackJobs jobs) 
   }
 }
 
+// 32 entries of a contraction's powers of two (DOzScale).  A launch of a few CTAs whose time is
+// its latency, hence 32 warps each: where the elements of an entry are contiguous a warp takes
+// an entry, else a lane does.
+__global__ void __launch_bounds__(1024) oz_scale_kernel(const __grid_constant__ OzScaleJobs jobs) {
+  __shared__ int top[32];
+  chain_wait();
+  chain_next();
+  const int jb = jobs.n > 1 && (int)blockIdx.x >= jobs.job[0].ntasks;
+  const OzScaleJob& job = jobs.job[jb];
+  const DOzScale t = job.tasks[blockIdx.x - (jb ? jobs.job[0].ntasks : 0)];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < 32) top[threadIdx.x] = 0;
+  __syncthreads();
+  for (int b = t.b0; b < t.b1; ++b) {
+    const DOzScaleBlock bl = job.blocks[b];
+    const bool by_lane = bl.istride == 1;
+    const int i = t.i0 + (by_lane ? lane : warp);
+    int m = 0;
+    if (i < t.dim) {
+      const double* p = job.src + bl.off + (long long)i * bl.istride;
+#pragma unroll 4
+      for (int l = by_lane ? warp : lane; l < bl.len; l += 32)
+        m = max(m, __double2hiint(p[(long long)l * bl.lstride]) & 0x7fffffff);
+    }
+    if (!by_lane) m = __reduce_max_sync(0xffffffffu, m);
+    if (m != 0 && (by_lane || lane == 0)) atomicMax(&top[by_lane ? lane : warp], m);
+  }
+  __syncthreads();
+  const int i = t.i0 + (int)threadIdx.x;
+  if (threadIdx.x >= 32 || i >= t.dim) return;
+  const int m = top[threadIdx.x];
+  const int e = m == 0 ? -127 : min(max((m >> 20) - 1022, -127), 127);
+  for (int r = 0; r < t.repeat; ++r) job.out[t.out + r * t.dim + i] = (int8_t)e;
+}
+
 }  // namespace
+
+void launch_oz_scale(const OzScaleJobs& jobs, cudaStream_t st) {
+  int n = 0;
+  for (int i = 0; i < jobs.n; ++i) n += jobs.job[i].ntasks;
+  if (n > 0) launch_chained(oz_scale_kernel, dim3(n), 1024, 0, st, jobs);
+}
 
 void launch_gemm_oz(const OzGemmArgs& a, cudaStream_t st) {
   if (a.nctas <= 0) return;
@@ -645,7 +715,7 @@ void launch_oz_pack(const OzPackJobs& jobs, cudaStream_t st) {
   int n = 0;
   for (int i = 0; i < jobs.n; ++i) n += jobs.job[i].npacks;
   if (n <= 0) return;
-  launch_chained(oz_pack_kernel, dim3(n), 256, 0, st, jobs);
+  launch_chained(jobs.job[0].scales ? oz_pack_kernel<true> : oz_pack_kernel<false>, dim3(n), 256, 0, st, jobs);
 }
 
 }  // namespace mpsxx

@@ -22,7 +22,7 @@ int slices(int k) { return (k + kOzTileK - 1) / kOzTileK; }
 // 128-row tile, column operands: across 32-row tiles).  segs_of(lo, hi) appends the segments
 // of rows [lo, hi).
 template <class F>
-void pack_rows(OzOperand& o, int rows, int k, bool row_operand, F segs_of) {
+void pack_rows(OzOperand& o, int rows, int k, int scale, bool row_operand, F segs_of) {
   const int nks = slices(k), log2 = row_operand ? 7 : 5, tile = 1 << log2, last = (rows - 1) / tile;
   const int tail = row_operand ? oz_tile_rows(rows, last) : oz_tail_cols(rows, last);
   const int most = std::min(kOzPackRows, std::max(8, kOzPackElems / (nks * kOzTileK) / 8 * 8));
@@ -43,6 +43,7 @@ void pack_rows(OzOperand& o, int rows, int k, bool row_operand, F segs_of) {
     pk.tile_log2 = log2;
     pk.last = last;
     pk.tail = tail;
+    pk.scale = scale;
     o.h_packs.push_back(pk);
     r0 += n;
   }
@@ -51,8 +52,8 @@ void pack_rows(OzOperand& o, int rows, int k, bool row_operand, F segs_of) {
 }
 
 // Every used block by itself.  tiled: the blocks' places in a tiled source.
-void pack_blocks(OzOperand& o, const Tensor& t, const std::vector<View>& view, bool row_operand,
-                 const std::vector<DOzTiled>* tiled = nullptr) {
+void pack_blocks(OzOperand& o, const Tensor& t, const std::vector<View>& view, const std::vector<int>& scale,
+                 bool row_operand, const std::vector<DOzTiled>* tiled = nullptr) {
   o.base.assign(view.size(), -1);
   o.exp0.assign(view.size(), 0);
   o.nks.assign(view.size(), 0);
@@ -62,7 +63,7 @@ void pack_blocks(OzOperand& o, const Tensor& t, const std::vector<View>& view, b
     o.base[s] = o.bytes;
     o.exp0[s] = o.rows;
     o.nks[s] = slices(v.k);
-    pack_rows(o, v.rows, v.k, row_operand, [&](int lo, int hi) {
+    pack_rows(o, v.rows, v.k, scale[s], row_operand, [&](int lo, int hi) {
       if (tiled == nullptr) {
         o.h_segs.push_back(DOzSeg{t.offsets[s] + int64_t(lo) * v.rstride, 0, hi - lo, v.rstride, v.kstride});
         return;
@@ -79,10 +80,50 @@ void pack_blocks(OzOperand& o, const Tensor& t, const std::vector<View>& view, b
   }
 }
 
+// The powers of two of a plan's contractions, one array per sector of the balancing index (and
+// size of the index before it): its tasks and blocks, and the first entry by block slot of A
+// and B.  Returns the number of entries; the arrays end at multiples of 16.
+int balance(OzGemm& og, const OzBalance& bal, const Tensor& a, const Tensor& b, std::vector<int>& sa, std::vector<int>& sb,
+            std::vector<DOzScaleBlock>& blocks) {
+  int n = 0;
+  const Tensor& of = bal.of;
+  std::vector<std::vector<DOzScaleBlock>> by_sector(of.sh.dshape[bal.axis].size());
+  for (size_t s = 0; s < of.tags.size(); ++s) {
+    int idx[kMaxRank], d[kMaxRank];
+    of.sh.index(of.tags[s], idx);
+    of.block_dims(static_cast<int32_t>(s), d);
+    if (d[0] > 0 && d[1] > 0)
+      by_sector[idx[bal.axis]].push_back(bal.axis == 0 ? DOzScaleBlock{of.offsets[s], d[1], d[1], 1}
+                                                       : DOzScaleBlock{of.offsets[s], d[0], 1, d[1]});
+  }
+  std::map<std::pair<int, int>, int> first;  // (sector, size of the index before)
+  auto slots = [&](const Tensor& t, int axis, int w, std::vector<int>& out) {
+    out.assign(t.tags.size(), 0);
+    for (size_t s = 0; s < t.tags.size(); ++s) {
+      int idx[kMaxRank];
+      t.sh.index(t.tags[s], idx);
+      const int sector = idx[axis], repeat = w < 0 ? 1 : t.sh.dshape[w][idx[w]], dim = t.sh.dshape[axis][sector];
+      if (dim <= 0 || repeat <= 0) continue;
+      const auto at = first.emplace(std::make_pair(sector, repeat), n);
+      out[s] = at.first->second;
+      if (!at.second) continue;
+      const int b0 = static_cast<int>(blocks.size());
+      if (sector < static_cast<int>(by_sector.size()) && of.sh.dshape[bal.axis][sector] == dim)
+        blocks.insert(blocks.end(), by_sector[sector].begin(), by_sector[sector].end());
+      for (int i0 = 0; i0 < dim; i0 += 32)
+        og.h_scale_tasks.push_back(DOzScale{n, dim, repeat, i0, b0, static_cast<int>(blocks.size())});
+      n += (dim * repeat + 15) / 16 * 16;
+    }
+  };
+  slots(a, bal.axis_a, bal.w_a, sa);
+  slots(b, bal.axis_b, bal.w_b, sb);
+  return n;
+}
+
 }  // namespace
 
-void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a, const Tensor& b, bool tiled_out,
-                   const OzGemm* from, const GemmPlan* from_plan) {
+void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a, const Tensor& b, const OzBalance& bal,
+                   bool tiled_out, const OzGemm* from, const GemmPlan* from_plan) {
   og.clear();
   // operand blocks as rows x K
   std::vector<View> va(a.tags.size()), vb(b.tags.size());
@@ -126,15 +167,23 @@ void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a,
   const std::vector<View>& vrb = og.swap ? va : vb;
   auto slot_a = [&](int p) { return og.swap ? g.pair_b_slot[p] : g.pair_a_slot[p]; };
   auto slot_b = [&](int p) { return og.swap ? g.pair_a_slot[p] : g.pair_b_slot[p]; };
-  pack_blocks(og.b, rb, vrb, false);
+  std::vector<DOzScaleBlock> scale_blocks;
+  std::vector<int> sa, sb;  // by block slot: first power of two of the block's contraction
+  const int nscales = balance(og, bal, a, b, sa, sb, scale_blocks);
+  const std::vector<int>& sra = og.swap ? sb : sa;
+  const std::vector<int>& srb = og.swap ? sa : sb;
+  og.a.sign = og.swap ? -bal.sign_a : bal.sign_a;
+  og.b.sign = -og.a.sign;
+  pack_blocks(og.b, rb, vrb, srb, false);
   std::vector<DOzPair> pairs;
   std::vector<int64_t> row_map;
   if (!single) {
-    pack_blocks(og.a, ra, vra, true, from != nullptr ? &place : nullptr);
+    pack_blocks(og.a, ra, vra, sra, true, from != nullptr ? &place : nullptr);
     pairs.resize(g.h_pairs.size());
     for (size_t p = 0; p < pairs.size(); ++p) {
       const int32_t as = slot_a(static_cast<int>(p)), bs = slot_b(static_cast<int>(p));
-      if (og.a.nks[as] != og.b.nks[bs]) throw Error(kInternal, "sliced gemm plan: operand packing mismatch");
+      if (og.a.nks[as] != og.b.nks[bs] || sra[as] != srb[bs])
+        throw Error(kInternal, "sliced gemm plan: operand packing mismatch");
       pairs[p] = DOzPair{og.a.base[as], og.b.base[bs], og.a.exp0[as], og.b.exp0[bs], og.a.nks[as], 0};
     }
     make_tiles(g, kOzTileM, kOzTileN, og.h_tiles, og.h_reduce, og.nslots, kOzTargetTiles);
@@ -179,14 +228,14 @@ void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a,
       }
       size_t j0 = 0;  // first task that reaches the next rows, and its first panel row
       int first = 0;
-      pack_rows(o, R, vc.k, true, [&](int lo, int hi) {
+      pack_rows(o, R, vc.k, srb[kv.first], true, [&](int lo, int hi) {
         while (j0 < kv.second.size() && first + vra[slot_a(g.h_tasks[kv.second[j0]].p0)].rows <= lo)
           first += vra[slot_a(g.h_tasks[kv.second[j0++]].p0)].rows;
         int at = first;
         for (size_t j = j0; j < kv.second.size() && at < hi; ++j) {
           const int32_t as = slot_a(g.h_tasks[kv.second[j]].p0);
           const View& v = vra[as];
-          if (v.k != vc.k) throw Error(kInternal, "sliced gemm plan: panel shapes differ");
+          if (v.k != vc.k || sra[as] != srb[kv.first]) throw Error(kInternal, "sliced gemm plan: panel shapes differ");
           const int x = std::max(at, lo), y = std::min(at + v.rows, hi);
           if (x < y)
             o.h_segs.push_back(DOzSeg{ra.offsets[as] + int64_t(x - at) * v.rstride, x - lo, y - x, v.rstride, v.kstride});
@@ -228,7 +277,11 @@ void build_oz_gemm(Context& ctx, OzGemm& og, const GemmPlan& g, const Tensor& a,
   }
   og.h_tiles.swap(sorted);
   const std::vector<int> none{0};
+  const std::vector<int8_t> zeros(nscales, 0);
   Upload up;
+  up.add(og.scale_tasks, og.h_scale_tasks);
+  up.add(og.scale_blocks, scale_blocks);
+  up.add(og.scales, zeros);
   up.add(og.tiles, og.h_tiles);
   up.add(og.cta_ptr, og.h_cta_ptr);
   up.add(og.pairs_tiled, pairs_tiled);
@@ -299,13 +352,24 @@ void oz_pack(Context& ctx, const std::vector<OzSource>& what) {
   OzPackJobs jobs{};
   for (const OzSource& w : what) {
     OzOperand& o = *w.o;
-    jobs.job[jobs.n++] = OzPackJob{o.packs.get(), o.segs.get(), w.src, o.digits, o.exps, o.flag.get(), static_cast<int>(o.h_packs.size()), o.seq + 1};
+    jobs.job[jobs.n++] = OzPackJob{o.packs.get(), o.segs.get(), w.src, o.digits, o.exps, o.flag.get(),
+                                   static_cast<int>(o.h_packs.size()), o.seq + 1,
+                                   w.balance ? w.balance->scales.get() : nullptr, o.sign};
   }
   launch_oz_pack(jobs, ctx.stream);
   for (const OzSource& w : what) {
     ++w.o->seq;
     w.o->cut = true;
   }
+  ctx.kernel_launches += 1;
+}
+
+void oz_scale(Context& ctx, const std::vector<std::pair<OzGemm*, const double*>>& what) {
+  OzScaleJobs jobs{};
+  for (const auto& w : what)
+    jobs.job[jobs.n++] = OzScaleJob{w.first->scale_tasks.get(), w.first->scale_blocks.get(), w.second,
+                                    w.first->scales.p, static_cast<int>(w.first->h_scale_tasks.size())};
+  launch_oz_scale(jobs, ctx.stream);
   ctx.kernel_launches += 1;
 }
 
