@@ -877,7 +877,9 @@ int mpsxx_sigma_device_time(mpsxx_context* ctx, const mpsxx_tensor* lopr, const 
   return guard([&] {
     need(reps > 0 && seconds != nullptr, "bad arguments");
     Context& c = ctx_of(ctx);
-    *seconds = sigma_device_time(c, ten(lopr), ten(ropr), ten(wfn), ten_mut(sgv), reps);
+    const double s = sigma_device_time(c, ten(lopr), ten(ropr), ten(wfn), ten_mut(sgv), reps);
+    check_device_error(c);
+    *seconds = s;
   });
 }
 
