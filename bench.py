@@ -121,6 +121,34 @@ def barrier(ws):
         dist.barrier()
 
 
+REQUIRED = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "config", "gpu_launches", "e2e", "clocks")
+
+
+def bench_line(out: dict, limit: int = 3000) -> str:
+    """The result as one line of at most `limit` characters: what a reader of the line needs,
+    then as much of the rest as fits, without its nested parts (the whole goes to stderr)."""
+
+    def short(x, depth):
+        if isinstance(x, float):
+            return float(f"{x:.6g}")
+        if isinstance(x, dict):
+            return {k: short(v, depth - 1) for k, v in x.items()
+                    if not isinstance(v, (dict, list, tuple)) or depth > 1 or (isinstance(v, (list, tuple)) and not v)}
+        if isinstance(x, (list, tuple)):
+            return [short(v, depth - 1) for v in x[:4]]
+        return x
+
+    line = {k: short(out[k], 2) if isinstance(out[k], dict) else out[k] for k in REQUIRED if k in out}
+    for k in out:
+        if k in line:
+            continue
+        more = {**line, k: short(out[k], 1 if isinstance(out[k], dict) else 2)}
+        if len(json.dumps(more)) <= limit:
+            line = more
+    return json.dumps(line)
+
+
 def job_tflops(ws: int, flops_per_rank_step: float, step_s: float) -> float:
     """Whole-job throughput of replicas: every rank does one step's work, the job's
     step time is the slowest rank's (already maxed over ranks)."""
@@ -984,7 +1012,8 @@ def main():
             "clocks": clk.summary(),
             "section_seconds": {k: round(v, 1) for k, v in sections.items()},
         }
-        print(json.dumps(out), flush=True)
+        print("details: " + json.dumps(out), file=sys.stderr, flush=True)
+        print(bench_line(out), flush=True)
     barrier(ws)
 
 
