@@ -201,7 +201,12 @@ void* Arena::take(size_t bytes, cudaStream_t st) {
   if (p_) cudaFree(p_);  // (waits for the work that uses it; not cached: every bond would leave a size)
   p_ = nullptr;
   cap_ = 0;
-  p_ = block_cache().get(bytes + bytes / 8, st, &cap_);
+  try {
+    p_ = block_cache().get(bytes + bytes / 8, st, &cap_);
+  } catch (const Error& e) {
+    if (e.code != kAlloc) throw;
+    p_ = block_cache().get(bytes, st, &cap_);
+  }
   st_ = st;
   return p_;
 }
@@ -1511,8 +1516,8 @@ static bool sigma_run_oz(Context& ctx, SigmaPlan& p, const DTensor& L, const DTe
   const OzGemm *bal1 = balanced ? &p.o1 : nullptr, *bal2 = balanced ? &p.o2 : nullptr;
   if (balanced) oz_scale(ctx, {{&p.o1, psi}, {&p.o2, psi}});
   std::vector<OzSource> pack{{&p.o1.b, psi, bal1}};
-  if (!p.o1.a.cut) pack.push_back({&p.o1.a, L.d, bal1});
-  if (!p.o2.b.cut) pack.push_back({&p.o2.b, R.d, bal2});
+  if (balanced || !p.o1.a.cut) pack.push_back({&p.o1.a, L.d, bal1});
+  if (balanced || !p.o2.b.cut) pack.push_back({&p.o2.b, R.d, bal2});
   oz_pack(ctx, pack);
   run_oz_gemm(ctx, p.o1, p.s1, 1.0, L.d, psi, scr, true);
   oz_pack(ctx, {{&p.o2.a, scr, bal2}});

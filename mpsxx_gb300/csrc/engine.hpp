@@ -286,7 +286,7 @@ struct SplitGemm {
 struct OzOperand {
   uint8_t* digits = nullptr;  // in the context's arena, for the length of a call
   int* exps = nullptr;        // one exponent per packed row
-  bool cut = false;           // the digits are those of the call's operand
+  bool cut = false;           // the digits are those of the call's operand, as it is
   std::vector<int64_t> base;  // per block slot: byte offset of its tile grid (-1: not packed)
   std::vector<int> exp0, nks;  // per block slot: first exponent, K slices
   std::vector<DOzPack> h_packs;

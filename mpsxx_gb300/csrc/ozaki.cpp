@@ -314,7 +314,7 @@ bool oz_reserve(Context& ctx, const std::vector<OzGemm*>& gs, const std::functio
       }
       part = std::max(part, g->partial_bytes());
     }
-    size_t need = (held ? 0 : digits) + (ctx.gemm_part.cap < part ? part : 0);
+    size_t need = (held || ctx.oz_mem.capacity() >= digits ? 0 : digits) + (ctx.gemm_part.cap < part ? part : 0);
     if (scratch.buf && scratch.buf->cap < scratch.bytes) need += scratch.bytes;
     if (need > kOzSmallBytes) {
       size_t free_b = 0, total_b = 0;
@@ -359,7 +359,7 @@ void oz_pack(Context& ctx, const std::vector<OzSource>& what) {
   launch_oz_pack(jobs, ctx.stream);
   for (const OzSource& w : what) {
     ++w.o->seq;
-    w.o->cut = true;
+    w.o->cut = w.balance == nullptr;
   }
   ctx.kernel_launches += 1;
 }

@@ -161,7 +161,7 @@ def test_memory_of_the_digits():
     used.append(fake.fake_used())
     # a tensor for which there is room only where the digits were
     fake.fake_limit(fake.fake_used())
-    n = 7 * (bonds[0][0].nnz + bonds[0][1].nnz)  # half of L's and R's digits
+    n = 14 * (bonds[0][0].nnz + bonds[0][1].nnz)  # L's and R's digits
     t = core.Tensor.create(ctx, (0, 0), [[(0, 0)]], [[n // 8]])
     short = product(bonds[0])
     fake.fake_limit(0)
