@@ -1676,8 +1676,8 @@ int* device_err_flag(Context& ctx) {
   return ctx.err_dev;
 }
 
-// 32 mapped host doubles of the context (the line after its error flag): *host as the host
-// sees them; returned as the device does.
+// 32 mapped host doubles of the context, 64 bytes after its error flag: *host as the host sees
+// them; returned as the device does.
 double* device_host_sums(Context& ctx, double** host) {
   int* dev = device_err_flag(ctx);
   *host = reinterpret_cast<double*>(ctx.err_host) + 8;

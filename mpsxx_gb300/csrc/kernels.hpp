@@ -194,8 +194,6 @@ void launch_fingerprints(const PrintJobs& jobs, int njobs, unsigned long long* s
 constexpr int kOzTileM = 128, kOzTileN = 32, kOzTileK = 16, kOzDigits = 7;
 constexpr int kOzGroupSteps = 10;     // K slices summed in one FP32 accumulation (exact up to 160)
 constexpr int kOzMaxExponent = 480;   // rows of magnitudes outside 2^-480 .. 2^480 flag their operand
-constexpr uint32_t kOzTileABytes = kOzDigits * kOzTileM * kOzTileK * 2;
-constexpr uint32_t kOzTileBBytes = kOzDigits * kOzTileN * kOzTileK * 2;
 __host__ __device__ constexpr int oz_tile_rows(int rows, int tm) {
   return rows - tm * 128 >= 128 ? 128 : (rows - tm * 128 + 7) / 8 * 8;
 }
@@ -345,7 +343,7 @@ void launch_eig_factors(const double* G, const double* w, int d, int k, int tran
 // (destinations with dst_off < 0 are skipped and leave their g untouched).
 void launch_adjoint_scatter(const DScatterDst* dsts, int ndst, const DScatterSrc* srcs, const double* Y,
                             const double* src, double* g, cudaStream_t st);
-// G[e] = sum_{k = ptr[e]}^{ptr[e+1]-1} g[idx[k]], summed in index order.
+// G[e] = sum_{k = ptr[e]}^{ptr[e+1]-1} g[idx[k]], in a fixed order (lanes in turn, then a tree).
 void launch_segment_sum(const int* ptr, const int* idx, const double* g, int ne, double* G, cudaStream_t st);
 void launch_diag(const DDiagTile* tiles, int ntiles, const DDiagTask* tasks, const DDiagPair* pairs, const double* L,
                  const double* R, double* out, cudaStream_t st);

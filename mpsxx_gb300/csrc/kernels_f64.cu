@@ -191,11 +191,11 @@ __global__ void copy_kernel(const DCopy* __restrict__ tasks, const double* __res
 // The sub-blocks tile the result, which is written once.  One warp per sub-block, its lanes
 // over consecutive elements, so that a source is read in whole lines and few lanes idle: the
 // FP64 pipe bounds the kernel (one multiply-add per contribution, 15 clocks of an SM per warp;
-// a leading coefficient of 1 costs none, and whether it is one is asked of the integer pipe:
-// with a comparison of doubles per source the calls below took 1357, 1221 and 279 us).
-// Elements per lane and CTAs per SM, QC n=20 M=512 forward (424 M contributions, 1.2 GB) /
-// backward / n=14 M=256, us: 3 x 32 and 4 1009 / 965 / 205, 3 and 5 1066 / 949 / 219, 4 and 6
-// 1150 / 993 / 238, 4 and 4 1018 / 1001 / 213, 2 and 5 1106 / 945 / 219.
+// a leading coefficient of 1 costs none, and whether it is one is asked of the integer pipe,
+// since a comparison of doubles is work for the FP64 pipe too).  Three elements per lane and four
+// CTAs per SM: 1009 us at QC n=20 M=512 forward (424 M contributions, 1.2 GB), 965 backward, 205
+// at n=14 M=256; two to four elements and four to six CTAs are at most 2 % faster in one of
+// these and 4 to 14 % slower in another.
 // Where there are too few sub-blocks to fill the chip, gridDim.y warps share one, in turn by
 // the 32 kScatterUnroll elements (see launch_scatter).
 constexpr int kScatterUnroll = 3;
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256) diag_kernel(const DDiagTile* __restrict__
   const int x = threadIdx.x & (w - 1), y = threadIdx.x >> tl.log2w;
   auto gather = [&](int p0, double* s) {
     const int np = min(kDiagPairs, t.p1 - p0);
-    // a warp takes four pairs, their loads in flight together
+    // a warp takes two pairs, their loads in flight together
     const int q0 = threadIdx.x >> 5;
     DDiagPair pr[kDiagPairs / 8];
 #pragma unroll

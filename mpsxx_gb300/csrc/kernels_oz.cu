@@ -431,9 +431,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_oz_kernel(const OzGemmArgs g
         double* dst = g.C + tk.c_off + (g.swap ? (int64_t)n0 * tk.ldc + r : (int64_t)r * tk.ldc + n0);
         const int64_t cs = g.swap ? tk.ldc : 1;
         // all old values before the first store: the compiler cannot tell that the columns do
-        // not overlap, and eight loads that waited for one another held the epilogue up (a
-        // Hubbard M=512 gradient, whose two such products took 135 us each: 617 -> 458 us; 434
-        // where nothing is added to)
+        // not overlap, and a load after each store would wait for it (a Hubbard M=512 gradient
+        // with its two products written that way took 617 us instead of 415)
         double old[EPI_COLS] = {};
         if (!g.assign)
 #pragma unroll
@@ -503,11 +502,11 @@ __device__ __forceinline__ unsigned long long biased56(double x, int e1022) {
 // (k ND + p) tile_rows 32 bytes.  A thread holds 8 consecutive K of a row per item, so that a warp
 // reads whole sectors and its stores fill 128-byte lines; up to kHold items stay in registers
 // between the two steps, what a long row has beyond is read again (from L2).  HBM moves 8 + 14
-// bytes per element; the integer pipe works about 45 instructions on one, which is why the
-// digits are cut by byte permutes and one FP32 addition each.  Both meet in the middle (HBM 65 %,
-// issue 50 %), so that warps in flight decide: four CTAs an SM (64 registers) against three, 2254 ->
-// 2199 us for a renormalisation at QC n=20 M=512 and 7.88 -> 7.68 ms for its H_eff*psi; five with one
-// item held lose it again to the second reads (2394 us, 7.97 ms).
+// bytes per element; the integer pipe works about 50 instructions on one (45 without powers of
+// two), which is why the digits are cut by byte permutes and one FP32 addition each.  Neither is
+// saturated (HBM 65 %, issue 50 %): warps in flight decide.  Four CTAs an SM (64 registers) against
+// three, and against five with one item held, whose second reads cost more: 7.68, 7.88, 7.97 ms
+// for H_eff*psi at QC n=20 M=512 (unbalanced).
 constexpr int kHold = 2;
 template <bool kScaled>
 __global__ void __launch_bounds__(256, 4) oz_pack_kernel(const __grid_constant__ OzPackJobs jobs) {
