@@ -998,7 +998,7 @@ static void pack_into(Context& ctx, Packed& P, const DTensor& t) {
 // Operators are packed once per (layout, data version).  One whose device pointer the caller
 // holds may hold other data in every call: its fingerprint is taken, and it is packed anew
 // where that is not the packed data's.  A product at QC n=20 M=512 / Hubbard M=256: 1.44 ms /
-// 73 us with operators known to be unchanged, 1.81 / 82 with fingerprints (the reading of both
+// 73 us with operators known to be unchanged, 1.81 / 79 with fingerprints (the reading of both
 // operators: 0.36 ms at the copy bandwidth), 4.3 / 99 where they are packed in every call.
 // The constructor queues the fingerprints and packs what is known to be other data; finish()
 // waits for the fingerprints and packs what they show to be.  In between the product may run

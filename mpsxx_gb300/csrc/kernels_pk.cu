@@ -660,8 +660,8 @@ void launch_pack(const DPack* packs, int npacks, const double* src, uint8_t* dst
 void launch_fingerprints(const PrintJobs& jobs, int njobs, unsigned long long* sums, cudaStream_t st) {
   int64_t n = 1;
   for (int j = 0; j < njobs; ++j) n = n < jobs.n[j] ? jobs.n[j] : n;
-  // two elements a thread at least, eight CTAs an SM at most
-  const int64_t want = (n + 511) / 512;
+  // eight elements a thread at least (each CTA adds to the same sums), eight CTAs an SM at most
+  const int64_t want = (n + 2047) / 2048;
   launch_kernel(fingerprint_kernel, dim3(want < 152 * 8 ? want : 152 * 8, njobs), 256, 0, st, jobs, sums);
 }
 

@@ -96,17 +96,19 @@ int balance(OzGemm& og, const OzBalance& bal, const Tensor& a, const Tensor& b, 
       by_sector[idx[bal.axis]].push_back(bal.axis == 0 ? DOzScaleBlock{of.offsets[s], d[1], d[1], 1}
                                                        : DOzScaleBlock{of.offsets[s], d[0], 1, d[1]});
   }
-  std::map<std::pair<int, int>, int> first;  // (sector, size of the index before)
+  std::map<int, std::vector<int>> first;  // by size of the index before: first entry by sector (-1: none)
   auto slots = [&](const Tensor& t, int axis, int w, std::vector<int>& out) {
     out.assign(t.tags.size(), 0);
+    const int64_t nsec = t.sh.nsec(axis);
     for (size_t s = 0; s < t.tags.size(); ++s) {
-      int idx[kMaxRank];
-      t.sh.index(t.tags[s], idx);
-      const int sector = idx[axis], repeat = w < 0 ? 1 : t.sh.dshape[w][idx[w]], dim = t.sh.dshape[axis][sector];
+      const int sector = static_cast<int>(t.tags[s] / t.sh.stride[axis] % nsec), dim = t.sh.dshape[axis][sector];
+      const int repeat = w < 0 ? 1 : t.sh.dshape[w][t.tags[s] / t.sh.stride[w] % t.sh.nsec(w)];
       if (dim <= 0 || repeat <= 0) continue;
-      const auto at = first.emplace(std::make_pair(sector, repeat), n);
-      out[s] = at.first->second;
-      if (!at.second) continue;
+      std::vector<int>& f = first[repeat];
+      if (f.empty()) f.assign(nsec, -1);
+      out[s] = f[sector] < 0 ? n : f[sector];
+      if (f[sector] >= 0) continue;
+      f[sector] = n;
       const int b0 = static_cast<int>(blocks.size());
       if (sector < static_cast<int>(by_sector.size()) && of.sh.dshape[bal.axis][sector] == dim)
         blocks.insert(blocks.end(), by_sector[sector].begin(), by_sector[sector].end());
