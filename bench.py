@@ -143,8 +143,9 @@ def bench_line(out: dict, limit: int = 3000) -> str:
     for k in out:
         if k in line:
             continue
-        more = {**line, k: short(out[k], 1 if isinstance(out[k], dict) else 2)}
-        if len(json.dumps(more)) <= limit:
+        part = short(out[k], 1 if isinstance(out[k], dict) else 2)
+        more = {**line, k: part}
+        if part not in ({}, []) and len(json.dumps(more)) <= limit:
             line = more
     return json.dumps(line)
 
