@@ -67,8 +67,8 @@ class Context:
         check(lib().mpsxx_context_set_device_timeout(self.h, int(timeout_ns)))
 
     def set_fp64_route(self, min_flops: float = -1.0):
-        """FP64 products of at least ``min_flops`` run on the tensor cores (error-free
-        slicing), smaller ones on the FP64 pipe; negative: the default, inf: none."""
+        """FP64 products of at least ``min_flops`` run on the tensor cores (operands sliced
+        into digits), smaller ones on the FP64 pipe; negative: the default, inf: none."""
         check(lib().mpsxx_context_set_fp64_route(self.h, float(min_flops)))
 
     def set_plan_cache(self, max_plans: int = 512):
